@@ -421,3 +421,30 @@ def test_relu2_gate_prologue_is_bit_identical(backend, codec, n, k, planes, m):
     with pytest.raises(errors.InvalidInput, match="not combined"):
         backend.norm_linear_forward_dev(resident, torch.from_numpy(gate).cuda(), got, relu2_up=torch.from_numpy(up).cuda(),
                                         norm_weight=torch.ones(k, device="cuda"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
+@pytest.mark.parametrize("k,planes", [(256, 1), (512, 1), (768, 1), (1280, 2), (768, 3), (2304, 3)])
+def test_tensor_core_tiles_at_their_edges(backend, codec, k, planes):
+    """Every token tile (32, 64, 128, 256) at its first and last token and one past it, with rows whose
+    tile-planes start on every 4-byte residue of a 16-byte line, a ragged last row tile, and as few
+    tile columns as there can be: int32 group sums and outputs against the oracle.  Group sums are
+    exact; an output is at most 54 fp32 additions, each within 2^-24 of the partial sum, behind a
+    product and in front of another one: 1e-5 relative leaves more than twice that."""
+    import torch
+    n = 133
+    prod, orac = uniform_pair(n, k, planes, seed=k + planes)
+    resident = backend.upload_salt_v2(prod, codec)
+    backend.reserve(resident, 300)
+    for m in (9, 32, 33, 64, 65, 128, 129, 256, 257):
+        x = make_activations(m, k, seed=m, bf16=True)
+        x_dev = torch.from_numpy(x).cuda().to(torch.bfloat16)
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        dump = torch.zeros(m, n, k // 128, planes, dtype=torch.int32, device="cuda")
+        backend.forward_dev(resident, x_dev, y, a8=True, acc_dump=dump)
+        torch.cuda.synchronize()
+        backend.check()
+        want, want_dump, _ = orc.a8_linear(orac, x, dump=True)
+        assert np.array_equal(dump.cpu().numpy(), want_dump[..., :planes]), m
+        assert rel_l2(y.cpu().numpy(), want) <= 1e-5, m
