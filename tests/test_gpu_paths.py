@@ -448,3 +448,28 @@ def test_tensor_core_tiles_at_their_edges(backend, codec, k, planes):
         want, want_dump, _ = orc.a8_linear(orac, x, dump=True)
         assert np.array_equal(dump.cpu().numpy(), want_dump[..., :planes]), m
         assert rel_l2(y.cpu().numpy(), want) <= 1e-5, m
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group", [64, 128])
+@pytest.mark.parametrize("n,k", [(9, 37), (11, 31 * 64 + 1), (17, 32 * 64 - 1), (5, 33 * 128 + 3), (8, 64 * 128 + 5)])
+def test_exact_kernel_where_its_chunks_of_segments_end(backend, group, n, k):
+    """Rows whose scale-group segments just fill, just exceed and several times exceed the 32 segments
+    that are staged at a time, with every offset of a row inside its group: the oracle's bits."""
+    from tritium_b200.format import SaltV2Tensor
+    rng = np.random.default_rng(n * k + group)
+    tiles, tail = -(-n * k // 256), n * k % 256
+    trits = np.zeros((tiles, 3, 256), np.int8)
+    trits[:, :2] = rng.integers(-1, 2, (tiles, 2, 256), dtype=np.int8)
+    trits[-1, :, tail:] = 0
+    gpt = 256 // group
+    scales = np.zeros((tiles, 3, 4), np.uint16)
+    scales[:, :2, :gpt] = (0.02 * np.abs(rng.standard_normal((tiles, 2, gpt))) + 1e-3).astype(np.float16).view(np.uint16)
+    scales[-1, :, -(-tail // group):] = 0
+    prod = SaltV2Tensor("w", n, k, np.full(tiles, 2, np.uint8), trits, scales, group)
+    orac = orc.Tensor(n, k, group, prod.plane_count, prod.trits, prod.scales)
+    resident = backend.upload_salt_v2(prod, SaltV2Codec.B3)
+    for m in (1, 3, 4, 5):
+        x = make_activations(m, k, seed=m)
+        got = backend.salt_v2_forward_exact(resident, x, m).output
+        assert np.array_equal(got.view(np.uint32), orc.matmul(orac, x).view(np.uint32)), m
