@@ -195,7 +195,7 @@ def measure_prefill(torch, backend, weights, m: int, codec_name: str, steps: int
             "ops_per_call": ops, "workload": f"c2_3plane_k2560_n6912_{codec_name}_m{m}", "out_dtype": "bf16",
             "l2_policy": f"weights rotate over {len(weights)} copies; activations stay L2-resident as they would after the previous layer",
             "roofline": {"bound": "tensor", "achieved": tops, "peak": peak, "unit": "TOPS", "frac": tops / peak,
-                         "peak_kind": kind, "frac_of_nominal_4500": tops / 4500.0, "kernel": "prefill_kernel"}}
+                         "peak_kind": kind, "frac_of_nominal_4500": tops / 4500.0, "kernel": "gemm_kernel"}}
 
 
 def measure_single_layer(torch, backend, weights, x_dev, m: int, layer_bytes: int, steps: int, stream, pdl_flag: int) -> dict:
