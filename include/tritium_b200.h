@@ -276,6 +276,10 @@ tb_status tb_backend_check(tb_backend* backend, void* stream);
  * reports TB_TIMEOUT, and the context stays usable.  Nothing faults, traps or spins without a
  * limit.  The hook disarms itself after that one call. */
 tb_status tb_backend_inject_wait_timeout(tb_backend* backend, uint32_t enable);
+/* Test hook, no counterpart in the reference, needs no device: the check every tensor-core launch of
+ * `m` tokens makes of the kernel it is about to launch.  TB_OK when a kernel compiled to `registers`
+ * registers per thread has enough of them for its warps' shares, TB_BACKEND when it would wait for ever. */
+tb_status tb_gemm_registers_check(uint32_t m, uint32_t registers);
 
 /* ------------------------------------------------------------------ trait path (1 plane, per-channel scale)
  * TernaryBackend::mpgemm (crates/tritium-spec/src/lib.rs:200-215; host crates/tritium-cuda/src/cuda/backend.rs:7175-7315)

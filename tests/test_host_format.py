@@ -347,3 +347,17 @@ def test_device_layout_leaves_small_and_unaligned_shapes_alone():
         got_p, got_s, info = mixed_small.device_layout(codec)
         assert np.array_equal(got_p, payload) and np.array_equal(got_s, scales)
         assert info["codec"] == int(codec) and not info["recoded"] and not info["counts_from_map"] and info["planes_uniform"] == 0
+
+
+# ------------------------------------------------------------------ launch checks that need no device
+@pytest.mark.parametrize("m,allotted", [(9, 80), (32, 80), (33, 80), (64, 80), (65, 80), (128, 80), (129, 96), (4096, 96)])
+def test_tensor_core_launch_is_refused_when_the_registers_do_not_go_round(m, allotted):
+    """The kernel's warps trade registers with setmaxnreg, whose request waits without a limit when the
+    pool is short.  A launch therefore looks at what the compiler allotted: the count of the launch
+    bounds passes, eight less per thread (the hardware's step) is too little, and a count above the
+    epilogue's share would turn its request for more into one for fewer."""
+    L = _lib.load()
+    errors.check(L.tb_gemm_registers_check(m, allotted))
+    for registers in (0, 40, allotted - 8, 168, 255, 1 << 20):
+        with pytest.raises(errors.BackendError, match="registers per thread"):
+            errors.check(L.tb_gemm_registers_check(m, registers))

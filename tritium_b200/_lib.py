@@ -29,7 +29,7 @@ EXPORTS = [
     "tb_fmt_resident_sizes", "tb_fmt_resident_build", "tb_fmt_package_write", "tb_fmt_tq2_pack_rows",
     "tb_fmt_quantize_act_int8", "tb_linear_forward_a8_static", "tb_backend_inject_wait_timeout",
     "tb_salt_v2_upload_reader", "tb_fmt_package_write_multi", "tb_fmt_package_extract", "tb_last_shape_mismatch", "tb_salt_v1_upload", "tb_tq1_upload",
-    "tb_fmt_device_layout",
+    "tb_fmt_device_layout", "tb_gemm_registers_check",
 ]
 
 
@@ -149,6 +149,7 @@ _SIGNATURES = {
     "tb_backend_reserve": (_ST, [_P, _P, _U32]),
     "tb_backend_check": (_ST, [_P, _P]),
     "tb_backend_inject_wait_timeout": (_ST, [_P, _U32]),
+    "tb_gemm_registers_check": (_ST, [_U32, _U32]),
     "tb_mpgemm": (_ST, [_P, _P, _P, _P, _U32, _U32, _U32, _P]),
     "tb_mpgemm_with_act_quant": (_ST, [_P, _P, _P, _P, _U32, _U32, _U32, _P]),
     "tb_stack_create": (_ST, [_P, _P, _P, _U32, _U32, _P]),

@@ -28,9 +28,10 @@
 // 34816 x 5120, 4096 tokens: 2,767 -> 1,768 us; 5120 x 17408, 16 tokens: 61 -> 37 us.  About a third of
 // that came from the outputs: a load in front of every store cost 270 clocks per output.
 //
-// TMEM: kAccBufs accumulators of kAccCols columns.  All waits are bounded; a timeout sets
+// TMEM: kAccBufs accumulators of kAccCols columns.  All waits on barriers are bounded; a timeout sets
 // TBF_WAIT_TIMEOUT and every role leaves its loop, the allocating warp frees TMEM, and the kernel
-// returns.  No TMA multicast is used.
+// returns.  The one wait that cannot be bounded, setmaxnreg's for registers, is ruled out before the
+// launch (Tile::pool_holds).  No TMA multicast is used.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -73,6 +74,19 @@ template <int TT> struct Tile {
   static constexpr uint32_t kTileBBytes = TT * 128;   // one slab of activations
   static constexpr size_t kSmem = 1024 + size_t(2 * kExpGroups) * kTileABytes + size_t(kStagesB) * 2 * kTileBBytes +
                                   size_t(kGroupWarps * kExpGroups) * kDepth * kStageBytes + size_t(kEpilogueWarps) * 32 * 4;
+  // Registers follow the work: each role sets its share per thread with setmaxnreg.  The pool is what the
+  // CTA got at launch, threads x the registers the compiler allotted (launch bounds: 96 per thread with
+  // 640 threads, 80 with 768), and a setmaxnreg.inc waits without limit for registers that the others
+  // have not given back, so the shares must add up to no more than the pool:
+  //   TT = 256:  128 x 40 (copy, MMA, idle) + 256 x 160 (epilogue) + 256 x 56 (expanders) = 60,416 <= 640 x 96
+  //   else:      128 x 40 + 256 x 112 + 384 x 72                                          = 61,440  = 768 x 80
+  // Another compiler or other flags may allot other counts: the launch asks the built kernel and is
+  // refused unless pool_holds (a share below the launch count is given back, one above it is drawn).
+  static constexpr int kControlRegs = 40, kEpilogueRegs = TT == 256 ? 160 : 112, kExpandRegs = TT == 256 ? 56 : 72;
+  static constexpr bool pool_holds(int launch_regs) {
+    return launch_regs >= kControlRegs && launch_regs >= kExpandRegs && launch_regs <= kEpilogueRegs &&
+           32 * (kFirstEpilogueWarp * kControlRegs + kEpilogueWarps * kEpilogueRegs + kGroupWarps * kExpGroups * kExpandRegs) <= kThreads * launch_regs;
+  }
 };
 
 constexpr uint32_t kSpin = 1u << 22;
@@ -785,17 +799,10 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
 }
 
 // ---------------------------------------------------------------- the kernel
-// Registers follow the work.  The pool is what the CTA got at launch (threads x kLaunchRegs), and the
-// shares below add up to no more than that, so that no setmaxnreg request can block:
-//   TT = 256:  640 x 96 = 61,440 >= 128 x 40 (copy, MMA, idle) + 256 x 160 (epilogue) + 256 x 56 (expanders)
-//   else:      768 x 80 = 61,440 >= 128 x 40 + 256 x 112 + 384 x 72 = 61,440
 template <int CODEC, int PLANES, int TT, bool DUMP>
 __global__ void __launch_bounds__(Tile<TT>::kThreads, 1) gemm_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q) {
   using T = Tile<TT>;
   constexpr uint32_t kTmemCols = T::kAccBufs * T::kAccCols;
-  constexpr int kControlRegs = 40, kEpilogueRegs = TT == 256 ? 160 : 112, kExpandRegs = TT == 256 ? 56 : 72;
-  constexpr int kLaunchRegs = TT == 256 ? 96 : 80;
-  static_assert(128 * kControlRegs + 256 * kEpilogueRegs + 128 * T::kExpGroups * kExpandRegs <= T::kThreads * kLaunchRegs, "register pool");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* tile_a = smem;
@@ -827,14 +834,14 @@ __global__ void __launch_bounds__(Tile<TT>::kThreads, 1) gemm_kernel(const Prefi
   const WaitCtx wctx{&abort_flag, p.status};
 
   if (warp < kFirstEpilogueWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kControlRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T::kControlRegs));
     if (warp == 0) copy_role<TT>(p, map_q, tiles, tile_b, b_full, b_empty, wctx, lane);
     else if (warp <= 2) mma_role<PLANES, TT>(p, tiles, tmem_base, warp - 1, tile_a, tile_b, a_full, a_empty, b_full, b_empty, acc_full, acc_empty, wctx);
   } else if (warp < kFirstExpandWarp) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(T::kEpilogueRegs));
     epilogue_role<PLANES, TT, DUMP>(p, tiles, tmem_base, warp, lane, saddr(scale_words) + (tid - 32 * kFirstEpilogueWarp) * 4, &combine_flag, acc_full, acc_empty, wctx);
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kExpandRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T::kExpandRegs));
     expander_role<CODEC, PLANES, TT>(p, tiles, warp - kFirstExpandWarp, lane, tile_a, stage, a_full, a_empty, wctx);
   }
   tc_fence_before();
@@ -882,44 +889,39 @@ Scratch carve(void* base, uint32_t m_pad, uint32_t k) {
   return s;
 }
 
-template <typename Kernel>
-cudaError_t launch_kernel(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const PrefillParams& pp, const CUtensorMap& map) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) return e;
-  // may start under the tail of the quantisation pre-pass (see tma_role)
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid; cfg.blockDim = dim3(unsigned(threads)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, pp, map);
-}
-
+// One instantiation of the kernel and what its launch needs.
+struct GemmKernel {
+  void (*fn)(PrefillParams, CUtensorMap);
+  int threads;
+  size_t smem;
+  bool (*pool_holds)(int);
+};
 template <int CODEC, int TT, bool DUMP>
-cudaError_t launch_planes(uint32_t planes, dim3 grid, cudaStream_t st, const PrefillParams& pp, const CUtensorMap& map) {
+GemmKernel kernel_of_planes(uint32_t planes) {
   using T = Tile<TT>;
-  if (planes == 1) return launch_kernel(gemm_kernel<CODEC, 1, TT, DUMP>, grid, T::kThreads, T::kSmem, st, pp, map);
-  if (planes == 2) return launch_kernel(gemm_kernel<CODEC, 2, TT, DUMP>, grid, T::kThreads, T::kSmem, st, pp, map);
-  return launch_kernel(gemm_kernel<CODEC, 3, TT, DUMP>, grid, T::kThreads, T::kSmem, st, pp, map);
+  return {planes == 1 ? gemm_kernel<CODEC, 1, TT, DUMP> : planes == 2 ? gemm_kernel<CODEC, 2, TT, DUMP> : gemm_kernel<CODEC, 3, TT, DUMP>,
+          T::kThreads, T::kSmem, T::pool_holds};
 }
-
-template <int CODEC>
-cudaError_t launch_shape(uint32_t tt, bool dump, uint32_t planes, dim3 grid, cudaStream_t st, const PrefillParams& pp, const CUtensorMap& map) {
-#define TB_TT_CASE(W) \
-  if (tt == W) return dump ? launch_planes<CODEC, W, true>(planes, grid, st, pp, map) : launch_planes<CODEC, W, false>(planes, grid, st, pp, map)
-  TB_TT_CASE(32);
-  TB_TT_CASE(64);
-  TB_TT_CASE(128);
-  TB_TT_CASE(256);
-#undef TB_TT_CASE
-  return cudaErrorInvalidValue;
+template <int CODEC, bool DUMP>
+GemmKernel kernel_of_tile(uint32_t tt, uint32_t planes) {
+  return tt == 32    ? kernel_of_planes<CODEC, 32, DUMP>(planes)
+         : tt == 64  ? kernel_of_planes<CODEC, 64, DUMP>(planes)
+         : tt == 128 ? kernel_of_planes<CODEC, 128, DUMP>(planes)
+                     : kernel_of_planes<CODEC, 256, DUMP>(planes);
+}
+GemmKernel kernel_of(int codec, uint32_t tt, uint32_t planes, bool dump) {
+  if (codec == tbf::kB3) return dump ? kernel_of_tile<tbf::kB3, true>(tt, planes) : kernel_of_tile<tbf::kB3, false>(tt, planes);
+  return dump ? kernel_of_tile<tbf::kD2, true>(tt, planes) : kernel_of_tile<tbf::kD2, false>(tt, planes);
 }
 
 }  // namespace
 
 bool tb_prefill_supported(const tb_weights* w, uint32_t m) {
   return w->fast && m >= 1 && w->k >= 256 && encode_tiled_fn() != nullptr;
+}
+
+bool tb_prefill_registers_hold(uint32_t m, int launch_regs) {
+  return kernel_of(tbf::kB3, tile_tokens(m), 1, false).pool_holds(launch_regs);   // the same for every codec and plane count
 }
 
 size_t tb_prefill_scratch_bytes(const tb_weights* w, uint32_t m) {
@@ -934,6 +936,14 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   const uint32_t m_pad = pad_tokens(a.m), k = uint32_t(w->k);
   if (!a.scratch || a.scratch_bytes < tb_prefill_scratch_bytes(w, a.m)) return cudaErrorInvalidValue;
   const Scratch sc = carve(a.scratch, m_pad, k);
+  const uint32_t tt = tile_tokens(a.m);
+  const GemmKernel kernel = kernel_of(w->codec, tt, w->uniform_planes, a.acc_dump != nullptr);
+  cudaFuncAttributes built;
+  cudaError_t err = cudaFuncGetAttributes(&built, kernel.fn);
+  if (err != cudaSuccess) return err;
+  if (!kernel.pool_holds(built.numRegs)) return cudaErrorInvalidConfiguration;   // its setmaxnreg would wait for ever
+  err = cudaFuncSetAttribute(kernel.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kernel.smem));
+  if (err != cudaSuccess) return err;
 
   QuantParams qp{};
   qp.x = a.x; qp.act_scale_in = a.act_scale_in; qp.act_absmax_in = a.act_absmax_in;
@@ -947,14 +957,13 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   // up to two rows per SM: wide CTAs, for the latency of one row; beyond that several rows share an SM
   if (m_pad <= 2u * uint32_t(sm_count)) prefill_quant_kernel<1024><<<m_pad, 1024, 0, stream>>>(qp);
   else prefill_quant_kernel<256><<<m_pad, 256, 0, stream>>>(qp);
-  cudaError_t err = cudaGetLastError();
+  err = cudaGetLastError();
   if (err != cudaSuccess) return err;
 
   // activations as a 2-D int8 tensor [m_pad rows][k bytes]; a box is one slab of one token tile
   CUtensorMap map;
   const cuuint64_t dims[2] = {k, m_pad};
   const cuuint64_t strides[1] = {k};
-  const uint32_t tt = tile_tokens(a.m);
   const cuuint32_t box[2] = {128, tt};
   const cuuint32_t elem[2] = {1, 1};
   if (encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, sc.qperm, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -972,8 +981,13 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
     if (!a.tile_counters) return cudaErrorInvalidValue;
     pp.partial = sc.partial; pp.tile_counters = a.tile_counters;
   }
-  const dim3 grid(std::min<uint32_t>(pp.n_tiles * pp.m_tiles * pp.splits, uint32_t(sm_count)));
-  const bool dump = a.acc_dump != nullptr;
-  return w->codec == tbf::kB3 ? launch_shape<tbf::kB3>(tt, dump, w->uniform_planes, grid, stream, pp, map)
-                              : launch_shape<tbf::kD2>(tt, dump, w->uniform_planes, grid, stream, pp, map);
+  // may start under the tail of the quantisation pre-pass (see copy_role)
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min<uint32_t>(pp.n_tiles * pp.m_tiles * pp.splits, uint32_t(sm_count)));
+  cfg.blockDim = dim3(unsigned(kernel.threads)); cfg.dynamicSmemBytes = kernel.smem; cfg.stream = stream;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel.fn, pp, map);
 }

@@ -739,6 +739,14 @@ extern "C" tb_status tb_backend_reserve(tb_backend* b, const tb_weights* w, uint
   return reserve_prefill(b, w, max_m);
 }
 
+extern "C" tb_status tb_gemm_registers_check(uint32_t m, uint32_t registers) {
+  clear_error();
+  if (!m) return tb_fail(TB_INVALID_INPUT, "a launch has at least one token");
+  if (registers > 255 || !tb_prefill_registers_hold(m, int(registers)))
+    return tb_fail(TB_BACKEND, "a tensor-core kernel of " + std::to_string(registers) + " registers per thread cannot share them out among its warps");
+  return TB_OK;
+}
+
 extern "C" tb_status tb_salt_v2_gather_rows(tb_backend* b, const tb_weights* w, const uint32_t* rows, size_t count, float* out) {
   clear_error();
   if (tb_status s = check_handles(b, w)) return s;

@@ -203,6 +203,8 @@ struct PrefillArgs {
   uint32_t* tile_counters = nullptr;     // 256 zeroed words (few-token launches split K and count the splits of a tile in)
 };
 bool tb_prefill_supported(const tb_weights* w, uint32_t m);
+// Whether the launch for `m` tokens accepts a kernel that was compiled to `launch_regs` registers per thread.
+bool tb_prefill_registers_hold(uint32_t m, int launch_regs);
 size_t tb_prefill_scratch_bytes(const tb_weights* w, uint32_t m);
 cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t stream);
 
