@@ -451,6 +451,37 @@ def test_tensor_core_tiles_at_their_edges(backend, codec, k, planes):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [24, 200])
+@pytest.mark.parametrize("dtype", ["bf16", "f32", "int8"])
+def test_unaligned_activations_in_front_of_the_tensor_cores(backend, m, dtype):
+    """The quantisation pre-pass reads eight activations per load where the rows start on 16-byte
+    boundaries, and one by one elsewhere: a pointer one element past a boundary gives the same bits."""
+    import torch
+    n, k = 80, 768
+    prod, orac = uniform_pair(n, k, 3, seed=13)
+    resident = backend.upload_salt_v2(prod, SaltV2Codec.B3)
+    backend.reserve(resident, m)
+    t = {"bf16": torch.bfloat16, "f32": torch.float32, "int8": torch.int8}[dtype]
+    x = make_activations(m, k, seed=4, bf16=dtype == "bf16")
+    q, s = orc.quantize_act_int8(x, m, k)
+    values = torch.from_numpy(np.asarray(q, np.float32).reshape(m, k) if dtype == "int8" else x).cuda().to(t)
+    scale = torch.from_numpy(np.asarray(s, np.float32)).cuda() if dtype == "int8" else None
+    flat = torch.zeros(m * k + 16, dtype=t, device="cuda")
+    outs = []
+    for start in (0, 1):
+        shifted = flat[start:start + m * k].view(m, k)
+        shifted.copy_(values)
+        assert (shifted.data_ptr() % 16 == 0) == (start == 0)
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        backend.forward_dev(resident, shifted, y, a8=True, act_scale=scale)
+        torch.cuda.synchronize()
+        backend.check()
+        outs.append(y)
+    assert torch.equal(outs[0], outs[1])
+    assert rel_l2(outs[1].cpu().numpy(), orc.a8_linear(orac, x, dump=False)[0]) <= 1e-5
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("group", [64, 128])
 @pytest.mark.parametrize("n,k", [(9, 37), (11, 31 * 64 + 1), (17, 32 * 64 - 1), (5, 33 * 128 + 3), (8, 64 * 128 + 5)])
 def test_exact_kernel_where_its_chunks_of_segments_end(backend, group, n, k):

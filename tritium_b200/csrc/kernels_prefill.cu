@@ -223,7 +223,7 @@ __host__ __device__ constexpr uint32_t d2_trit_of_slot(uint32_t s) {
   const uint32_t quad = s >> 2, e = s & 3;   // quad 4w + i = slot i of the word's four bytes
   return 16 * (quad >> 2) + 4 * e + (quad & 3);
 }
-template <int CODEC> struct SlotTable {
+template <int CODEC> struct alignas(16) SlotTable {
   uint8_t trit[256];
   constexpr SlotTable() : trit{} {
     for (uint32_t s = 0; s < 256; ++s) trit[s] = uint8_t(CODEC == tbf::kB3 ? b3_trit_of_slot(s) : d2_trit_of_slot(s));
@@ -239,8 +239,9 @@ template <int CODEC> constexpr bool slots_are_a_permutation() {
   return true;
 }
 static_assert(slots_are_a_permutation<tbf::kB3>() && slots_are_a_permutation<tbf::kD2>(), "k-slot order");
-__constant__ SlotTable<tbf::kB3> c_b3_slots{};
-__constant__ SlotTable<tbf::kD2> c_d2_slots{};
+// In global memory: every lane wants another entry, which constant memory would hand out one at a time.
+__device__ const SlotTable<tbf::kB3> d_b3_slots{};
+__device__ const SlotTable<tbf::kD2> d_d2_slots{};
 
 // ---------------------------------------------------------------- quantisation pre-pass
 struct QuantParams {
@@ -248,7 +249,7 @@ struct QuantParams {
   const float* relu2_up;   // squared-ReLU gate (x fp32): activation = (max(x, 0)^2) * relu2_up; null = none
   int8_t* qperm; float* ascale;
   uint32_t m, k, x_dtype, codec;
-  uint32_t vec;            // rows (and the gate's) start on 16-byte boundaries: eight values per load
+  uint32_t vec;            // x starts on a 16-byte boundary, and so does each row: eight values per load (the gate is read value by value)
   uint32_t* status;
 };
 
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(THREADS) prefill_quant_kernel(const QuantParam
     if (tid == 0) p.ascale[t] = 0.f;
     return;
   }
-  if (tid < 256) slots[tid] = p.codec == tbf::kB3 ? c_b3_slots.trit[tid] : c_d2_slots.trit[tid];
+  if (tid < 64) reinterpret_cast<uint32_t*>(slots)[tid] = __ldg(reinterpret_cast<const uint32_t*>(p.codec == tbf::kB3 ? d_b3_slots.trit : d_d2_slots.trit) + tid);
   const size_t row = size_t(t) * p.k;
   float scale_q = 1.f;
   if (p.x_dtype != TB_I8) {
@@ -954,8 +955,10 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   qp.qperm = sc.qperm; qp.ascale = sc.ascale;
   qp.vec = (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0;   // k is a multiple of 256: every row starts like the first
   qp.m = a.m; qp.k = k; qp.x_dtype = uint32_t(a.x_dtype); qp.codec = uint32_t(w->codec); qp.status = a.status;
-  // up to two rows per SM: wide CTAs, for the latency of one row; beyond that several rows share an SM
-  if (m_pad <= 2u * uint32_t(sm_count)) prefill_quant_kernel<1024><<<m_pad, 1024, 0, stream>>>(qp);
+  // Up to two rows per SM that take 256 threads more than one step: wide CTAs, for the latency of one row
+  // (16 tokens: 2,560 columns 5.0 against 5.7 us, 17,408 columns 9.0 against 14.1; but 1,024 columns 4.8
+  // against 4.4).  Else several rows share an SM (512 tokens of 2,560 columns: 6.6 against 8.4 us).
+  if (m_pad <= 2u * uint32_t(sm_count) && k > 2048) prefill_quant_kernel<1024><<<m_pad, 1024, 0, stream>>>(qp);
   else prefill_quant_kernel<256><<<m_pad, 256, 0, stream>>>(qp);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
