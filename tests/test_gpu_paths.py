@@ -427,11 +427,12 @@ def test_relu2_gate_prologue_is_bit_identical(backend, codec, n, k, planes, m):
 @pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
 @pytest.mark.parametrize("k,planes", [(256, 1), (512, 1), (768, 1), (1280, 2), (768, 3), (2304, 3)])
 def test_tensor_core_tiles_at_their_edges(backend, codec, k, planes):
-    """Every token tile (32, 64, 128, 256) at its first and last token and one past it, with rows whose
-    tile-planes start on every 4-byte residue of a 16-byte line, a ragged last row tile, and as few
-    tile columns as there can be: int32 group sums and outputs against the oracle.  Group sums are
+    """Token tiles of 32, 64 and 128 (one and several) at their first and last token and one past it, with
+    rows whose tile-planes start on every 4-byte residue of a 16-byte line, a ragged last row tile, and as
+    few tile columns as there can be: int32 group sums and outputs against the oracle.  Group sums are
     exact; an output is at most 54 fp32 additions, each within 2^-24 of the partial sum, behind a
-    product and in front of another one: 1e-5 relative leaves more than twice that."""
+    product and in front of another one: 1e-5 relative leaves more than twice that.  The kernel without
+    the dump is another instantiation: its outputs (fp32, bf16, with a residual) follow bit for bit."""
     import torch
     n = 133
     prod, orac = uniform_pair(n, k, planes, seed=k + planes)
@@ -448,6 +449,49 @@ def test_tensor_core_tiles_at_their_edges(backend, codec, k, planes):
         want, want_dump, _ = orc.a8_linear(orac, x, dump=True)
         assert np.array_equal(dump.cpu().numpy(), want_dump[..., :planes]), m
         assert rel_l2(y.cpu().numpy(), want) <= 1e-5, m
+        outputs_follow_without_the_dump(backend, resident, x_dev, y)
+
+
+def outputs_follow_without_the_dump(backend, resident, x_dev, y):
+    """The same call without the dump, in fp32, in bf16 and with a residual, against the dump form's fp32 outputs."""
+    import torch
+    y2, y16 = torch.full_like(y, float("nan")), torch.full_like(y, float("nan"), dtype=torch.bfloat16)
+    y3, residual = torch.full_like(y, float("nan")), torch.randn(y.shape, device="cuda")
+    backend.forward_dev(resident, x_dev, y2, a8=True)
+    backend.forward_dev(resident, x_dev, y16, a8=True)
+    backend.norm_linear_forward_dev(resident, x_dev, y3, residual=residual)
+    torch.cuda.synchronize()
+    backend.check()
+    assert torch.equal(y, y2) and torch.equal(y.to(torch.bfloat16), y16) and torch.equal(residual + y, y3), y.shape
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
+@pytest.mark.parametrize("k,planes", [(1280, 1), (1024, 2), (512, 3)])
+def test_wide_token_tiles_at_their_edges(backend, codec, k, planes):
+    """Token tiles of 256, which take more than four tile-planes per row and row tiles enough to fill the
+    GPU: 76 of them (the last one ragged) at one token more than a tile of 128 holds, at a full tile, and at
+    three tiles, where each CTA has several.  Sampled rows against the oracle, as in the test above."""
+    import torch
+    from gpu_common import oracle_rows, product_only, sample_rows
+    n = 9605
+    prod = product_only(n, k, planes, seed=k)
+    rows = sample_rows(n)
+    orac, resident = oracle_rows(prod, rows), backend.upload_salt_v2(prod, codec)
+    backend.reserve(resident, 700)
+    for m in (129, 256, 700):
+        x = make_activations(m, k, seed=m, bf16=True)
+        x_dev = torch.from_numpy(x).cuda().to(torch.bfloat16)
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        dump = torch.zeros(m, n, k // 128, planes, dtype=torch.int32, device="cuda")
+        backend.forward_dev(resident, x_dev, y, a8=True, acc_dump=dump)
+        torch.cuda.synchronize()
+        backend.check()
+        want, want_dump, _ = orc.a8_linear(orac, x, dump=True)
+        at = torch.from_numpy(rows).cuda()
+        assert np.array_equal(dump[:, at].cpu().numpy(), want_dump[..., :planes]), m
+        assert rel_l2(y[:, at].cpu().numpy(), want) <= 1e-5, m
+        outputs_follow_without_the_dump(backend, resident, x_dev, y)
 
 
 @pytest.mark.gpu

@@ -866,14 +866,29 @@ EncodeTiled encode_tiled_fn() {
   return fn;
 }
 
-// Token tile: one of 32, 64 or 128 tokens for that many tokens, else tiles of 256.
-uint32_t tile_tokens(uint32_t m) { return m <= 32 ? 32 : m <= 64 ? 64 : m <= 128 ? 128 : 256; }
-uint32_t pad_tokens(uint32_t m) { const uint32_t t = tile_tokens(m); return (m + t - 1) / t * t; }
+// Widest token tile that `m` tokens take, and the tokens padded to it (the rows of the scratch).
+uint32_t widest_tile(uint32_t m) { return m <= 32 ? 32 : m <= 64 ? 64 : m <= 128 ? 128 : 256; }
+uint32_t pad_tokens(uint32_t m) { const uint32_t t = widest_tile(m); return (m + t - 1) / t * t; }
+// Token tile: one of 32, 64 or 128 tokens for that many tokens; beyond that 256, or 128 where
+//   * the tiles of 128 still fit one wave, or take half as many waves again at most and a row has no more than
+//     40 tile-planes: a CTA is done with a 128-token tile in 0.65 to 0.7 of a 256-token tile's time (half
+//     the drain and outputs, three expander groups in place of two), longer rows at the upper end;
+//   * a row has no more than four tile-planes: the outputs then outweigh the sums, and the 256-token
+//     tile's unrolled output code is twice as long when it has to come from memory first.
+// Measured, tiles of 256 -> 128, us (caches flushed in front of each call): 512 x 1024, 1 plane, 256 tokens
+// 33.7 -> 19.5; 2560 x 2560, 3 planes, 256 tokens 62.6 -> 42.0; 6912 x 512, 1 plane, 2048 tokens 54.2 -> 48.0.
+// Where 256 stays: 6912 x 2560, 3 planes, 2048 tokens 165 against 194.
+uint32_t tile_tokens(const tb_weights* w, uint32_t m, uint32_t sm_count) {
+  if (m <= 128) return widest_tile(m);
+  const uint64_t n_tiles = (w->n + kRows - 1) / kRows, tile_planes = w->k / 256 * w->uniform_planes;
+  const auto waves = [&](uint32_t tt) { return (n_tiles * ((m + tt - 1) / tt) + sm_count - 1) / sm_count; };
+  const uint64_t half = waves(128), whole = waves(256);
+  return half == whole || (2 * half <= 3 * whole && tile_planes <= 40) || tile_planes <= 4 ? 128 : 256;
+}
 // K splits of an output tile: as many as keep every CTA of one wave busy, at most one per tile column.
 uint32_t splits_of(const tb_weights* w, uint32_t m, uint32_t sm_count) {
-  const uint32_t tt = tile_tokens(m), tpr = uint32_t(w->k / 256);
-  const uint32_t out_tiles = uint32_t((w->n + kRows - 1) / kRows) * (pad_tokens(m) / tt);
-  if (tt > 64 || out_tiles >= sm_count || out_tiles > kMaxSplitTiles) return 1;
+  const uint32_t tpr = uint32_t(w->k / 256), out_tiles = uint32_t((w->n + kRows - 1) / kRows);
+  if (m > 64 || out_tiles >= sm_count || out_tiles > kMaxSplitTiles) return 1;   // up to 64 tokens are one token tile
   return std::max(1u, std::min(std::min(sm_count / out_tiles, tpr), 8u));
 }
 
@@ -922,7 +937,7 @@ bool tb_prefill_supported(const tb_weights* w, uint32_t m) {
 }
 
 bool tb_prefill_registers_hold(uint32_t m, int launch_regs) {
-  return kernel_of(tbf::kB3, tile_tokens(m), 1, false).pool_holds(launch_regs);   // the same for every codec and plane count
+  return kernel_of(tbf::kB3, widest_tile(m), 1, false).pool_holds(launch_regs);   // the same for every codec and plane count
 }
 
 size_t tb_prefill_scratch_bytes(const tb_weights* w, uint32_t m) {
@@ -937,7 +952,7 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   const uint32_t m_pad = pad_tokens(a.m), k = uint32_t(w->k);
   if (!a.scratch || a.scratch_bytes < tb_prefill_scratch_bytes(w, a.m)) return cudaErrorInvalidValue;
   const Scratch sc = carve(a.scratch, m_pad, k);
-  const uint32_t tt = tile_tokens(a.m);
+  const uint32_t tt = tile_tokens(w, a.m, uint32_t(sm_count)), m_tiles = (a.m + tt - 1) / tt, rows = m_tiles * tt;   // rows <= m_pad
   const GemmKernel kernel = kernel_of(w->codec, tt, w->uniform_planes, a.acc_dump != nullptr);
   cudaFuncAttributes built;
   cudaError_t err = cudaFuncGetAttributes(&built, kernel.fn);
@@ -958,14 +973,14 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   // Up to two rows per SM that take 256 threads more than one step: wide CTAs, for the latency of one row
   // (16 tokens: 2,560 columns 5.0 against 5.7 us, 17,408 columns 9.0 against 14.1; but 1,024 columns 4.8
   // against 4.4).  Else several rows share an SM (512 tokens of 2,560 columns: 6.6 against 8.4 us).
-  if (m_pad <= 2u * uint32_t(sm_count) && k > 2048) prefill_quant_kernel<1024><<<m_pad, 1024, 0, stream>>>(qp);
-  else prefill_quant_kernel<256><<<m_pad, 256, 0, stream>>>(qp);
+  if (rows <= 2u * uint32_t(sm_count) && k > 2048) prefill_quant_kernel<1024><<<rows, 1024, 0, stream>>>(qp);
+  else prefill_quant_kernel<256><<<rows, 256, 0, stream>>>(qp);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
 
-  // activations as a 2-D int8 tensor [m_pad rows][k bytes]; a box is one slab of one token tile
+  // activations as a 2-D int8 tensor [rows][k bytes]; a box is one slab of one token tile
   CUtensorMap map;
-  const cuuint64_t dims[2] = {k, m_pad};
+  const cuuint64_t dims[2] = {k, rows};
   const cuuint64_t strides[1] = {k};
   const cuuint32_t box[2] = {128, tt};
   const cuuint32_t elem[2] = {1, 1};
@@ -978,7 +993,7 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   pp.ascale = sc.ascale;
   pp.y = a.y; pp.acc_dump = a.acc_dump; pp.row_scale = a.row_scale; pp.status = a.status; pp.residual = a.residual;
   pp.m = a.m; pp.m_pad = m_pad; pp.n = uint32_t(w->n); pp.k = k; pp.tpr = k / 256; pp.y_dtype = uint32_t(a.y_dtype);
-  pp.n_tiles = (pp.n + kRows - 1) / kRows; pp.m_tiles = m_pad / tt;
+  pp.n_tiles = (pp.n + kRows - 1) / kRows; pp.m_tiles = m_tiles;
   pp.splits = splits_of(w, a.m, uint32_t(sm_count));
   if (pp.splits > 1) {
     if (!a.tile_counters) return cudaErrorInvalidValue;
