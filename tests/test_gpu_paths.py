@@ -548,3 +548,82 @@ def test_exact_kernel_where_its_chunks_of_segments_end(backend, group, n, k):
         x = make_activations(m, k, seed=m)
         got = backend.salt_v2_forward_exact(resident, x, m).output
         assert np.array_equal(got.view(np.uint32), orc.matmul(orac, x).view(np.uint32)), m
+
+
+F32_MAX = float(np.finfo(np.float32).max)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group", [64, 128])
+@pytest.mark.parametrize("what", ["element", "scale", "running_sum"])
+@pytest.mark.parametrize("m,token", [(1, 0), (3, 1), (6, 5)])
+def test_exact_overflow_names_the_row_and_column_of_the_reference(backend, group, what, m, token):
+    """One row and one token leave the finite range, far behind the first 32 scale groups: at an element
+    in the middle of a segment, where a segment's sum meets its scale, or where the running sum takes the
+    second of two large contributions.  The message names what the oracle names."""
+    from tritium_b200.format import SaltV2Tensor
+    rng = np.random.default_rng(group)
+    n, k, row = 5, 40 * group + 7, 3
+    tiles, tail, gpt = -(-n * k // 256), n * k % 256, 256 // group
+    trits = np.zeros((tiles, 3, 256), np.int8)
+    trits[:, :2] = rng.integers(-1, 2, (tiles, 2, 256), dtype=np.int8)
+    scales = np.zeros((tiles, 3, 4), np.uint16)
+    scales[:, :2, :gpt] = (0.02 * np.abs(rng.standard_normal((tiles, 2, gpt))) + 1e-3).astype(np.float16).view(np.uint16)
+    first = 36 * group + group // 2
+    at = [first + i for i in range(6)] if what != "running_sum" else [first, first + group]
+    for r in range(n):           # the columns in question count in one row only
+        for c in at:
+            tile, local = divmod(r * k + c, 256)
+            trits[tile, :, local] = (1, 0, 0) if r == row else 0
+            if r == row and what != "element":
+                scales[tile, 0, local // group] = 0x7BFF if what == "scale" else 0x3C00
+    trits[-1, :, tail:] = 0
+    scales[-1, :, -(-tail // group):] = 0
+    prod = SaltV2Tensor("w", n, k, np.full(tiles, 2, np.uint8), trits, scales, group)
+    orac = orc.Tensor(n, k, group, prod.plane_count, prod.trits, prod.scales)
+    resident = backend.upload_salt_v2(prod, SaltV2Codec.B3)
+    x = make_activations(m, k, seed=m)
+    x[token, at] = {"element": F32_MAX / 3, "scale": F32_MAX / 1000, "running_sum": F32_MAX / 4 * 3}[what]
+    with pytest.raises(orc.OracleError) as e:
+        orc.matvec(orac, x[token])
+    assert e.value.row == row and e.value.column > 33 * group
+    with pytest.raises(errors.InvalidInput, match=f"output row {e.value.row} became non-finite at column {e.value.column}$"):
+        backend.salt_v2_forward_exact(resident, x, m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")], ids=["inf", "nan"])
+def test_exact_kernel_leaves_out_zero_trits_of_nonfinite_activations(backend, bad):
+    """Device pointers, bit-exact route: an activation that is not finite is reported, and it reaches only the
+    outputs of rows whose trits there are not all zero, and only those of its own token."""
+    import torch
+    n, k, m, token, column = 24, 33 * 64 + 5, 4, 2, 32 * 64 + 9
+    from tritium_b200.format import SaltV2Tensor
+    rng = np.random.default_rng(5)
+    tiles = -(-n * k // 256)
+    trits = np.zeros((tiles, 3, 256), np.int8)
+    trits[:, :2] = rng.integers(-1, 2, (tiles, 2, 256), dtype=np.int8)
+    scales = np.zeros((tiles, 3, 4), np.uint16)
+    scales[:, :2] = (0.02 * np.abs(rng.standard_normal((tiles, 2, 4))) + 1e-3).astype(np.float16).view(np.uint16)
+    tail = n * k % 256
+    trits[-1, :, tail:] = 0
+    scales[-1, :, -(-tail // 64):] = 0
+    prod = SaltV2Tensor("w", n, k, np.full(tiles, 2, np.uint8), trits, scales, 64)
+    resident = backend.upload_salt_v2(prod, SaltV2Codec.B3)
+    where = np.arange(n) * k + column
+    reached = trits[where // 256, :, where % 256].any(axis=1)
+    assert reached.any() and not reached.all()
+    x = make_activations(m, k, seed=1)
+    clean = x.copy()
+    clean[token, column] = 0
+    x[token, column] = bad
+    want = orc.matmul(orc.Tensor(n, k, 64, prod.plane_count, prod.trits, prod.scales), clean)
+    y = torch.full((m, n), 7.0, dtype=torch.float32, device="cuda")
+    backend.forward_dev(resident, torch.from_numpy(x).cuda(), y, a8=False, flags=_lib.TB_FWD_EXACT)
+    torch.cuda.synchronize()
+    with pytest.raises(errors.InvalidInput, match="non-finite"):
+        backend.check()
+    got, same = y.cpu().numpy(), np.ones((m, n), bool)
+    same[token, reached] = False
+    assert np.array_equal(got.view(np.uint32)[same], want.view(np.uint32)[same])
+    assert not np.isfinite(got[~same]).any()

@@ -68,7 +68,7 @@ __device__ __forceinline__ int trit_at(const uint8_t* base, uint32_t codec, uint
 // crates/tritium-cuda/kernels/tq2_0_add.cu:107-175): the only rounding left is the final one.
 //
 // acc + trit * x, one rounding: the product is exact, so this is the reference's ga +/- x.  A zero trit
-// adds a zero, which changes no bit: a sum that starts at +0 never becomes -0.
+// adds a zero, which changes no bit while x is finite: a sum that starts at +0 never becomes -0.
 __device__ __forceinline__ float acc_step(float a, float trit, float x) { return __fmaf_rn(trit, x, a); }
 __device__ __forceinline__ double acc_step(double a, float trit, float x) { return __fma_rn(double(trit), double(x), a); }
 template <typename Acc> __device__ __forceinline__ Acc acc_mul(Acc a, float b);
@@ -76,6 +76,38 @@ template <> __device__ __forceinline__ float acc_mul<float>(float a, float b) { 
 template <> __device__ __forceinline__ double acc_mul<double>(double a, float b) { return __dmul_rn(a, double(b)); }
 __device__ __forceinline__ float shfl_acc(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
 __device__ __forceinline__ double shfl_acc(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+
+// One output in the reference's own order, element by element (crates/tritium-cpu/src/salt_v2.rs:316-423): zero
+// trits are left out (0 x infinity is no zero), and `column` becomes the one at which the row leaves the
+// finite range: the element for a group sum, the segment's last column for its product with the scale
+// or the running sum.  One thread, for outputs that came out not finite.
+constexpr uint32_t kFinite = 0xffffffffu;
+template <typename Acc>
+__device__ __forceinline__ Acc row_in_order(const ExactParams& p, uint32_t row, uint32_t token, const uint16_t* lut, uint32_t& column) {
+  const uint32_t full_bytes = plane_bytes_dev(p.codec, 256), full_scales = 256u / p.group;
+  const float* x = p.x + uint64_t(token) * p.k;
+  const auto note = [&](Acc v, uint32_t col) { if (!isfinite(v) && column == kFinite) column = col; };
+  Acc acc = Acc(0);
+  for (uint32_t col = 0, len; col < p.k; col += len) {
+    const uint64_t c = uint64_t(row) * p.k + col, tile = c >> 8, rank = rank_of(p, tile);
+    const uint32_t local0 = uint32_t(c & 255), g = local0 / p.group, planes = planes_of(p, tile);
+    const uint32_t tlen = uint32_t(min(uint64_t(256), p.coeffs - (tile << 8)));
+    len = min((g + 1) * p.group - local0, p.k - col);
+    for (uint32_t q = 0; q < planes; ++q) {
+      const uint8_t* base = p.payload + rank * full_bytes + uint64_t(q) * plane_bytes_dev(p.codec, tlen);
+      Acc ga = Acc(0);
+      for (uint32_t e = 0; e < len; ++e) {
+        const int trit = trit_at(base, p.codec, local0 + e, lut);
+        if (trit == 0) continue;
+        ga = acc_step(ga, float(trit), x[col + e]);
+        note(ga, col + e);
+      }
+      acc = acc + acc_mul<Acc>(ga, __half2float(__ushort_as_half(p.scales[rank * full_scales + q * ((tlen + p.group - 1) / p.group) + g])));
+      note(acc, col + len - 1);
+    }
+  }
+  return acc;
+}
 
 // Activations of one chunk of segments in shared memory, [column][token], every scale group's columns
 // one position further: the lanes of a warp read columns a whole group apart, which would
@@ -109,8 +141,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) salt_v2_exact_kernel(cons
   Acc acc[kTokens];
 #pragma unroll
   for (int t = 0; t < kTokens; ++t) acc[t] = Acc(0);
-  bool bad = false;
-  uint32_t bad_col = 0;
 
   // Segment s of this row: boundaries are the row start, every tile-local group boundary, and
   // the row end.  first_boundary = distance from the row start to the next group boundary.
@@ -165,19 +195,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) salt_v2_exact_kernel(cons
           ga[3] = acc_step(ga[3], trit, xv.w);
         }
 #pragma unroll
-        for (int t = 0; t < kTokens; ++t) {
-          contrib[q][t] = acc_mul<Acc>(ga[t], scale);
-          if (!isfinite(ga[t]) && !bad) {
-            // a sum that left the finite range stays outside: find the column where it did
-            bad = true;
-            Acc again = Acc(0);
-            for (uint32_t e = 0; e < len; ++e) {
-              again = acc_step(again, float(trit_at(base, p.codec, local0 + e, lut)), p.x[uint64_t(m0 + t) * p.k + col0 + e]);
-              if (!isfinite(again)) { bad_col = col0 + e; break; }
-            }
-          }
-          if (!isfinite(contrib[q][t]) && !bad) { bad = true; bad_col = col0 + len - 1; }
-        }
+        for (int t = 0; t < kTokens; ++t) contrib[q][t] = acc_mul<Acc>(ga[t], scale);
       }
     }
     // ordered fold: segment ascending, plane ascending
@@ -197,13 +215,24 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) salt_v2_exact_kernel(cons
     }
   }
   if (!live) return;
+  // A sum that has left the finite range stays outside, so the end shows whether there was one.  Every lane
+  // holds the same sums; those in question are done again by one lane per token.
+  uint32_t again = 0;
 #pragma unroll
-  for (int t = 0; t < kTokens; ++t)
-    if (!isfinite(acc[t]) && !bad) { bad = true; bad_col = p.k - 1; }
-  if (__any_sync(0xffffffffu, bad)) {
-    if (bad && atomicOr(&p.status[TBS_FLAGS], TBF_NONFINITE_OUT) == 0) {
+  for (int t = 0; t < kTokens; ++t) again |= uint32_t(!isfinite(acc[t])) << t;
+  if (again) {
+    uint32_t column = kFinite;
+    Acc sum = Acc(0);
+    if ((again >> lane) & 1u) sum = row_in_order<Acc>(p, row, m0 + lane, lut, column);
+    const uint32_t failed = __ballot_sync(0xffffffffu, column != kFinite);
+    if (failed && lane == uint32_t(__ffs(failed)) - 1 && atomicOr(&p.status[TBS_FLAGS], TBF_NONFINITE_OUT) == 0) {
       p.status[TBS_INFO0] = row;
-      p.status[TBS_INFO1] = bad_col;
+      p.status[TBS_INFO1] = column;
+    }
+#pragma unroll
+    for (int t = 0; t < kTokens; ++t) {
+      const Acc v = shfl_acc(sum, t);
+      if ((again >> t) & 1u) acc[t] = v;
     }
   }
   if (lane == 0) {
