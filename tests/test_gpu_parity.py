@@ -588,3 +588,19 @@ def test_int8_path_of_other_layouts_is_bit_identical_to_cpu(backend, codec, ocod
     assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
     with pytest.raises(errors.UnsupportedFormat, match="accumulator dump"):
         backend.linear_forward_a8(resident, x, m, dump=True)
+
+
+@pytest.mark.parametrize("codec,k,planes,m", [
+    (SaltV2Codec.B3, 11520, 1, 1), (SaltV2Codec.B3, 12544, 1, 2), (SaltV2Codec.B3, 14080, 1, 1), (SaltV2Codec.D2, 10240, 1, 3),
+    (SaltV2Codec.D2, 13056, 1, 1), (SaltV2Codec.D2, 17408, 1, 1),
+])
+def test_decode_rings_that_fill_shared_memory(backend, codec, k, planes, m):
+    """Row lengths whose ring, tables and partial sums come within 2 KB of the shared memory a CTA can have:
+    the kernel's static shared memory (barriers, layer descriptors) has to fit beside them."""
+    n = 40
+    prod, orac = uniform_pair(n, k, planes, seed=k)
+    x = make_activations(m, k, seed=m)
+    want_y, want_acc, _ = orc.a8_linear(orac, x)
+    y, acc, _ = backend.linear_forward_a8(backend.upload_salt_v2(prod, codec), x, m, dump=True)
+    assert np.array_equal(acc, want_acc[:, :, :, :planes])
+    assert rel_l2(y, want_y) <= 1e-5

@@ -1190,8 +1190,11 @@ TableLayout table_layout(const tb_weights* w, uint32_t m_valid) {
   return t;
 }
 
-// Shared-memory layout for (weights, m); returns total bytes or 0 when it cannot fit.
-size_t layout(const tb_weights* w, uint32_t m, int max_smem, DecodeParams* p) {
+// Shared-memory layout for (weights, m); returns the dynamic bytes or 0 when it cannot fit beside the
+// kernel's static shared memory.
+constexpr uint32_t kStaticBytes = (2 * kMaxStages + 1 + 2 * kPartBufs) * 8 + 2 * 4 + kMaxGroupLayers * sizeof(TbLayerDesc) + 128;   // 128: alignment
+size_t layout(const tb_weights* w, uint32_t m, int max_smem_optin, DecodeParams* p) {
+  const int max_smem = max_smem_optin - int(kStaticBytes);
   const DecodePlan& pl = w->plan;
   const uint32_t planes = w->uniform_planes;
   const TableLayout tl = table_layout(w, m);
