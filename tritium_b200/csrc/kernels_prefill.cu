@@ -37,6 +37,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "tb_internal.h"
 
@@ -908,15 +909,20 @@ Scratch carve(void* base, uint32_t m_pad, uint32_t k) {
 // One instantiation of the kernel and what its launch needs.
 struct GemmKernel {
   void (*fn)(PrefillParams, CUtensorMap);
+  std::atomic<int>* regs;   // registers per thread it was built with, 0 until asked for: a fact of this library, the same on every device
   int threads;
   size_t smem;
   bool (*pool_holds)(int);
 };
+template <int CODEC, int PLANES, int TT, bool DUMP> std::atomic<int> g_built_regs{0};
+template <int CODEC, int PLANES, int TT, bool DUMP>
+GemmKernel kernel_instance() {
+  using T = Tile<TT>;
+  return {gemm_kernel<CODEC, PLANES, TT, DUMP>, &g_built_regs<CODEC, PLANES, TT, DUMP>, T::kThreads, T::kSmem, T::pool_holds};
+}
 template <int CODEC, int TT, bool DUMP>
 GemmKernel kernel_of_planes(uint32_t planes) {
-  using T = Tile<TT>;
-  return {planes == 1 ? gemm_kernel<CODEC, 1, TT, DUMP> : planes == 2 ? gemm_kernel<CODEC, 2, TT, DUMP> : gemm_kernel<CODEC, 3, TT, DUMP>,
-          T::kThreads, T::kSmem, T::pool_holds};
+  return planes == 1 ? kernel_instance<CODEC, 1, TT, DUMP>() : planes == 2 ? kernel_instance<CODEC, 2, TT, DUMP>() : kernel_instance<CODEC, 3, TT, DUMP>();
 }
 template <int CODEC, bool DUMP>
 GemmKernel kernel_of_tile(uint32_t tt, uint32_t planes) {
@@ -954,10 +960,14 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   const Scratch sc = carve(a.scratch, m_pad, k);
   const uint32_t tt = tile_tokens(w, a.m, uint32_t(sm_count)), m_tiles = (a.m + tt - 1) / tt, rows = m_tiles * tt;   // rows <= m_pad
   const GemmKernel kernel = kernel_of(w->codec, tt, w->uniform_planes, a.acc_dump != nullptr);
-  cudaFuncAttributes built;
-  cudaError_t err = cudaFuncGetAttributes(&built, kernel.fn);
-  if (err != cudaSuccess) return err;
-  if (!kernel.pool_holds(built.numRegs)) return cudaErrorInvalidConfiguration;   // its setmaxnreg would wait for ever
+  cudaError_t err = cudaSuccess;
+  int regs = kernel.regs->load(std::memory_order_relaxed);
+  if (!regs) {
+    cudaFuncAttributes built;
+    if ((err = cudaFuncGetAttributes(&built, kernel.fn)) != cudaSuccess) return err;
+    kernel.regs->store(regs = built.numRegs, std::memory_order_relaxed);
+  }
+  if (!kernel.pool_holds(regs)) return cudaErrorInvalidConfiguration;   // its setmaxnreg would wait for ever
   err = cudaFuncSetAttribute(kernel.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kernel.smem));
   if (err != cudaSuccess) return err;
 
