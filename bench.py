@@ -273,7 +273,7 @@ def measure_int8_peak(torch) -> dict | None:
 
 
 def measure_few_tokens(torch, backend, codec, stream, shapes=None, batches=(16, 32, 64), copies_cap: int = 0) -> dict:
-    """Batches of 9 to 64 tokens (batched decode): one call of the few-token tensor-core kernel per
+    """Batches of 9 to 64 tokens (batched decode): one call of the tensor-core kernel per
     linear against chained 4-token decode passes, on the benchmark's layer and on a 27B-class gate/up
     linear, weights rotating over copies larger than L2, eager calls (quantisation pre-pass included)."""
     from tritium_b200 import _lib
@@ -624,7 +624,7 @@ def run_b200(args) -> None:
 
     stream = torch.cuda.Stream()
     if args.only_few_tokens:
-        # profiling aid: the few-token tensor-core kernel alone, on the 27B-class gate/up linear
+        # profiling aid: the tensor-core kernel at few tokens alone, on the 27B-class gate/up linear
         print(json.dumps(measure_few_tokens(torch, backend, codec, stream, shapes=[("gate_up_27b_2plane", 34816, 5120, 2)],
                                             batches=(args.only_few_tokens,), copies_cap=3)), flush=True)
         return
@@ -835,7 +835,7 @@ def main() -> None:
     ap.add_argument("--skip-cpu", action="store_true")
     ap.add_argument("--prefill-m", type=int, default=2048, help="tokens of the tensor-core leg (0 = skip)")
     ap.add_argument("--only-prefill", action="store_true")
-    ap.add_argument("--only-few-tokens", type=int, default=0, metavar="M", help="profiling aid: only the few-token kernel at M tokens (9..64)")
+    ap.add_argument("--only-few-tokens", type=int, default=0, metavar="M", help="profiling aid: only the tensor-core kernel at M tokens (9..64)")
     ap.add_argument("--no-tp", action="store_true", help="skip the tensor-parallel decoder-stack leg")
     ap.add_argument("--tp-prefill-m", type=int, default=4096, help="tokens of the tensor-parallel prefill pass (0 = skip)")
     ap.add_argument("--tp-shape", default="27b", choices=["27b", "2b"], help="decoder whose linears the tensor-parallel leg runs")

@@ -470,9 +470,9 @@ def test_stack_host_call_matches_per_layer_calls(backend):
 def test_mixed_plane_counts_on_aligned_shapes_take_the_fast_kernels(backend, codec, m):
     """A tensor whose tiles hold one to three planes (a plane map with varying counts), on a shape
     the fast kernels take, is stored padded to three plane slots per tile with all-zero planes.
-    The int8 path then runs the decode, few-token and many-token kernels with the same exact
-    group sums (zero for a padded plane); the fp32 exact kernel still adds only each tile's true
-    planes and returns the reference's bits."""
+    The int8 path then runs the decode kernel and the tensor-core kernel at small and large token tiles
+    with the same exact group sums (zero for a padded plane); the fp32 exact kernel still adds only each
+    tile's true planes and returns the reference's bits."""
     n, k = 64, 768
     prod, orac = uniform_pair(n, k, 3, seed=91)
     tiles = n * k // 256

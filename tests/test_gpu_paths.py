@@ -356,7 +356,7 @@ def test_backend_freed_before_its_weights():
     (48, 19200, 512, 2),    # more row tiles than SMs: no split, several tiles per CTA
 ])
 def test_few_token_tensor_core_kernel_is_exact(backend, codec, m, n, k, planes):
-    """Batches of 9 to 64 tokens run one pass of the few-token tensor-core kernel (accumulator ring,
+    """Batches of 9 to 64 tokens run one pass of the tensor-core kernel with a tile of 32 or 64 (accumulator ring,
     sums in registers, K split over CTAs with a fixed-order combine).  The int32 group sums must be
     the oracle's bit for bit, with and without the dump, and two runs must give the same bits."""
     import torch
@@ -396,8 +396,8 @@ def test_few_token_tensor_core_kernel_is_exact(backend, codec, m, n, k, planes):
     (192, 1024, 2, 1),      # tables built in the decode kernel
     (160, 6912, 1, 4),      # the 2B-class down projection's width: preparation kernel
     (256, 2560, 3, 6),      # two passes
-    (256, 1536, 2, 40),     # few-token tensor-core kernel
-    (128, 1024, 1, 200),    # many-token kernel
+    (256, 1536, 2, 40),     # tensor-core kernel, one tile of 64 tokens
+    (128, 1024, 1, 200),    # two tiles of 128
 ])
 def test_relu2_gate_prologue_is_bit_identical(backend, codec, n, k, planes, m):
     """(max(gate, 0)^2) * up is computed where the activations are quantised; elementwise and

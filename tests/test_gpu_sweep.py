@@ -1,5 +1,5 @@
 """Seeded random sweep over shapes, token counts, codecs and options of the int8 linear: every
-route (decode passes, few-token and many-token tensor-core kernels; RMSNorm or squared-ReLU gate
+route (decode passes, tensor-core kernel at small and large token tiles; RMSNorm or squared-ReLU gate
 in front, residual behind; bf16 output) against the CPU oracle.  Temporaries are handed to the
 library and dropped at once on purpose: calls run on torch's current stream, so the allocator's
 stream-ordered reuse must be safe."""

@@ -11,8 +11,9 @@
 //     UMMA M = 128).  EXP groups work on consecutive tile-planes at once;
 //   * a copy warp loads the int8 activations of the tile column (B operand) by TMA from the scratch
 //     written by the quantisation pre-pass, already in the expanders' k-slot order;
-//   * one MMA warp issues four tcgen05.mma (kind::i8, N = TT, K = 32 each) per slab into a ring of
-//     TMEM accumulators; the first one overwrites, so nothing has to be stored to TMEM;
+//   * two MMA warps issue four tcgen05.mma (kind::i8, N = TT, K = 32 each) per slab into a ring of TMEM
+//     accumulators, one slab each of a 256-token tile's tile-planes, alternate tile-planes of a smaller
+//     tile; the first MMA of a slab overwrites, so nothing has to be stored to TMEM;
 //   * eight epilogue warps (one TMEM lane = one weight row per thread, half of the tile's tokens
 //     each) read a finished accumulator, hand it back, and add the slab's exact integer sums times
 //     the row's f16 group scale to fp32 running sums in their REGISTERS.
@@ -21,8 +22,10 @@
 // conversion and one multiply-add for each of its 32,768 sums (measured alone: 645 clocks with scalar
 // FFMA, 733 with packed FFMA2, whose register pairs cost moves).  Conversions, byte permutes and logic
 // share the ALU pipe at 2 clocks per warp: 423 such instructions per scheduler and slab, 847 of the
-// about 1,500 clocks a slab takes (ncu: 1,020 instructions per scheduler and slab, issue slots 64 %).
-// A smaller tile: the expansion, about 2,700 clocks per tile-plane and group, three groups at once.
+// about 1,580 clocks a slab takes (ncu: 1,060 instructions per scheduler and slab, issue slots 67 %).
+// A smaller tile: the expansion, three groups at once (5120 x 17408, 2 planes, 16 tokens, ncu with cold
+// caches: 59,500 clocks per CTA for 45 tile-planes, start, combine and outputs among them; issue
+// slots 70 %, DRAM 13 %).
 // Measured against the previous form (running sums and pre-loaded start values in TMEM, the
 // expanders' loads word by word), 3 planes, 6912 x 2560, 2048 tokens: 217 -> 147 us; 2 planes,
 // 34816 x 5120, 4096 tokens: 2,767 -> 1,768 us; 5120 x 17408, 16 tokens: 61 -> 37 us.  About a third of

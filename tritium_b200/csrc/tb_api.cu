@@ -451,8 +451,11 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
     fill_receipt(w, a.m, dtype_size(a.x_dtype), dtype_size(a.y_dtype), 0, ex.norm_weight ? 4 : 3, receipt);
     return TB_OK;
   }
-  // measured crossover (C2, 27B and 2B linears alike): two chained 4-token decode passes are level with
-  // one call of the few-token tensor-core kernel (about 25 us on C2), three passes are slower
+  // One or two chained decode passes (up to 4 or 8 tokens), else the tensor cores.  Measured with flushed
+  // caches, us, decode / tensor cores, at 4, 5 and 8 tokens: 6912 x 2560, 3 planes 23.5 / 23.5, 37.9 / 23.5,
+  // 33.8 / 23.5; 2560 x 2560, 1 plane 15.6 / 19.4, 27.6 / 19.4, 25.6 / 17.4; 34816 x 5120, 2 planes 48 / 60,
+  // 87 / 60, 87 / 60.  So one pass is level or faster; the limit of two passes was drawn when the
+  // tensor-core kernel took 25 us where it takes 20 now, and two passes lose by a third today.
   const bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags);
   uint32_t extra_launches = 0;
   // The decode kernel normalises inside its table builder.  Every other route (the tensor-core
@@ -933,6 +936,10 @@ extern "C" tb_status tb_stack_forward_dev(tb_stack* st, const void* x, tb_dtype 
       // [layer][m][n] bf16, whichever kernel family runs.
       const StackGroup& g = st->groups[gi];
       const tb_weights* w = st->layers[i];
+      // A grouped pass serves every layer with one launch.  Measured, us per layer, grouped passes / tensor
+      // cores, at 12, 16 and 20 tokens: 6912 x 2560, 3 planes 12.2 / 20.5, 16.2 / 20.6, 20.2 / 20.6; 2560 x 2560,
+      // 1 plane 3.3 / 14.5, 4.3 / 16.5, 5.3 / 15.8; but 13824 x 2560, 1 plane 12.2 / 14.5, 16.1 / 14.5, 20.1 / 14.5
+      // and 7168 x 5120, 2 planes 22.1 / 22.8, 29.1 / 22.8, 36.1 / 22.8: 16 is right for narrow layers, 12 for wide ones.
       const bool prefill = takes_tensor_cores(b, w, m, flags, 16);
       if (prefill) {
         for (size_t l = 0; l < g.count; ++l) {
