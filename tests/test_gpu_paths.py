@@ -12,7 +12,7 @@ from tritium_b200 import _lib, errors
 from tritium_b200.format import SaltV2Codec
 from tritium_b200.synth import bf16_bits_to_f32, f32_to_bf16_bits, make_activations
 
-from gpu_common import rel_l2, uniform_pair
+from gpu_common import exact_group_sums, rel_l2, uniform_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -421,6 +421,38 @@ def test_relu2_gate_prologue_is_bit_identical(backend, codec, n, k, planes, m):
     with pytest.raises(errors.InvalidInput, match="not combined"):
         backend.norm_linear_forward_dev(resident, torch.from_numpy(gate).cuda(), got, relu2_up=torch.from_numpy(up).cuda(),
                                         norm_weight=torch.ones(k, device="cuda"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
+@pytest.mark.parametrize("k,m", [(256, 1), (256, 4), (1024, 3), (1024, 4), (1280, 4), (2048, 2), (2304, 2), (4096, 1), (4096, 2), (4352, 1),
+                                 (4352, 2), (8192, 1), (8448, 1)])
+def test_activation_tables_where_their_passes_end(backend, codec, k, m):
+    """Tables built in the decode kernel: one (tile column, token) pair, a full pass of 16 and one more, the
+    largest number it takes and one more (then the preparation kernel).  fp32, bf16 and int8
+    activations (whole int8 range): int32 group sums equal to the oracle's, outputs within 1e-5."""
+    import torch
+    n = 20
+    prod, orac = uniform_pair(n, k, 1, seed=k + m)
+    resident = backend.upload_salt_v2(prod, codec)
+    x = make_activations(m, k, seed=m, bf16=True)
+    want, want_acc, _ = orc.a8_linear(orac, x)
+    acc = torch.full((m, n, k // 128, 1), 7, dtype=torch.int32, device="cuda")
+    y = torch.zeros(m, n, device="cuda")
+    for xt in (torch.from_numpy(x).cuda(), to_dev_bf16(x)):
+        backend.forward_dev(resident, xt, y, acc_dump=acc)
+        backend.check()
+        assert np.array_equal(acc.cpu().numpy(), want_acc[..., :1])
+        assert rel_l2(y.cpu().numpy(), want) <= 1e-5
+    q = np.random.default_rng(k).integers(-128, 128, (m, k)).astype(np.int8)
+    scale = torch.linspace(0.5, 1.5, m, device="cuda")
+    backend.forward_dev(resident, torch.from_numpy(q).cuda(), y, act_scale=scale, acc_dump=acc)
+    backend.check()
+    sums = exact_group_sums(prod.raw[0], q)
+    assert np.array_equal(acc.cpu().numpy(), sums)
+    per_group = prod.raw[1][0].astype(np.float16).astype(np.float64)   # as the artifact stores them
+    ref = (sums[..., 0] * per_group).sum(axis=2) * scale.double().cpu().numpy()[:, None]
+    assert rel_l2(y.cpu().numpy(), ref) <= 1e-5
 
 
 @pytest.mark.gpu

@@ -51,7 +51,6 @@ constexpr int kConsumerThreads = kWarps * 32;
 constexpr int kMaxStages = 4;
 constexpr int kPartBufs = 4;   // row blocks whose partial sums may wait for the combiner
 constexpr int kMaxGroupLayers = 128;   // layers of one grouped launch (descriptors live in shared memory)
-constexpr uint32_t kBuildStagingBytes = 32 * 272 + 8 * 16 + 16 + 128;   // fused prologue: quantised activations of one pass of pairs, absmax partials, 1/rms per token, the peers' absmax
 
 struct DecodeParams {
   const uint8_t* payload; const uint16_t* scales;   // single layer (layers == nullptr)
@@ -454,298 +453,316 @@ __global__ void __launch_bounds__(256) prepare_kernel(const PrepareParams p) {
   }
 }
 // ---------------------------------------------------------------- fused prologue
-// Eight elements of a row starting at element `idx` (a multiple of 8; rows are 16-byte aligned).
-__device__ __forceinline__ void load8(const void* x, uint32_t dtype, size_t idx, float (&v)[8]) {
-  if (dtype == TB_F32) {
-    const float4 a = reinterpret_cast<const float4*>(x)[idx / 4], b = reinterpret_cast<const float4*>(x)[idx / 4 + 1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else if (dtype == TB_BF16) {
-    const uint4 u = reinterpret_cast<const uint4*>(x)[idx / 8];
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
-  } else {
-    const uint2 u = reinterpret_cast<const uint2*>(x)[idx / 8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[i] = float(int(int8_t(u.x >> (8 * i))));
-      v[4 + i] = float(int(int8_t(u.y >> (8 * i))));
-    }
-  }
+// Four elements of a row starting at element `idx` (a multiple of 4; rows are 16-byte aligned).
+__device__ __forceinline__ void load4_f32(const float* x, size_t idx, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(x + idx);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
 
-// MMA number that consumes digit pair `pair` of the packed words of `slot` (words 4*slot .. 4*slot+3;
-// slot 3 of B3 is the bytewise MMA on word 12) for scale group `v`, or -1 when that combination holds
-// only zeros (the inverse of slot_of).
-template <int CODEC, bool DUAL> __device__ __forceinline__ int mma_of(uint32_t slot, uint32_t pair, uint32_t v) {
-  if (CODEC == tbf::kB3) {
-    if (DUAL) return slot < 3 ? int(slot * 3 + pair) : 9;
-    if (slot == 0) return v == 0 ? int(pair) : -1;
-    if (slot == 1) return int((v == 0 ? 3 : 6) + pair);
-    if (slot == 2) return v == 1 ? int(9 + pair) : -1;
-    return v == 1 ? 12 : -1;
-  }
-  if (DUAL) return int(slot * 2 + pair);
-  return (slot >> 1) == v ? int(slot * 2 + pair) : -1;
+// MMA number that consumes digit pair 0 of the packed words of `slot` (words 4*slot .. 4*slot+3; slot 3
+// of B3 is the bytewise MMA on word 12) for scale group `v`; the next pairs' MMAs follow it (the
+// inverse of slot_of).
+template <int CODEC, bool DUAL> __device__ __forceinline__ uint32_t first_mma_of(uint32_t slot, uint32_t v) {
+  if (CODEC == tbf::kB3) return DUAL ? slot * 3 : slot * 3 + (slot == 1 ? v * 3 : slot >= 2 ? 3 : 0);
+  return slot * 2;
 }
 
-constexpr uint32_t kChunkPairs = 32;    // (tile column, token) pairs quantised per pass of the table builder
-constexpr uint32_t kPairStride = 272;   // staged bytes per pair: 256 codes + zero padding (B3 digits 256..259)
+// A table builder's pass: the eight consumer warps hold kSteps half tiles (128 activations of one scale
+// group) each in registers, four activations per lane.
+constexpr uint32_t kSteps = 4;
+constexpr uint32_t kChunkPairs = kSteps * kWarps / 2;   // (tile column, token) pairs per pass
+constexpr uint32_t kPairStride = 272;                   // staged bytes per pair: 256 codes + padding (B3 digits 256..259)
+// staging of the builder in shared memory: codes | norm slots | absmax bits, 1/rms, code and output scales per token | peers' absmax
+constexpr uint32_t kStageSlots = kChunkPairs * kPairStride, kStageTokens = kStageSlots + kConsumerThreads * 4, kStagePeers = kStageTokens + 4 * 16,
+                   kBuildStagingBytes = kStagePeers + 8 * 16;
 
-__device__ __forceinline__ int sbyte(uint32_t w, int b) { return int(int8_t(w >> (8 * b))); }
+// What the builder needs before the activations are there: zero table entries, codes of zero behind
+// every pair, absmax of zero.  A following barrier of the consumers separates it from the builder.
+__device__ __forceinline__ void clear_tables(const DecodeParams& p, uint8_t* smem, uint32_t tid) {
+  for (uint32_t at = p.off_z + tid * 16; at < p.off_cinit; at += kConsumerThreads * 16) *reinterpret_cast<uint4*>(smem + at) = make_uint4(0, 0, 0, 0);
+  if (tid < kChunkPairs) *reinterpret_cast<uint32_t*>(smem + p.off_xq + tid * kPairStride + 256) = 0x80808080u;
+  if (tid < 4) reinterpret_cast<uint32_t*>(smem + p.off_xq + kStageTokens)[tid] = 0u;
+}
 
 // Builds this CTA's activation tables in shared memory (same contents as prepare_kernel writes to
 // global scratch): per-token absmax int8 quantisation of x, B-fragment entries, accumulator start
 // values, token scales.  Called by the eight consumer warps (tid 0..255).
 //
-// Work item of the entry construction = one packed word position w of one (tile column, token,
-// scale group): the 20 (B3) or 16 (D2) activations that meet the word's digits are five (four)
-// aligned 32-bit words of the staged codes, every one of them inside a single scale group; their
-// transformed values z = x_t - 3 x_(t-1) (B3; x_t for D2), split as 4*high + low, are the table
-// words of that position.  Items are independent, so the whole CTA works on them at once.
-// y = (x * inv) * w (or (1 + w)) for eight consecutive columns: the reference's rmsnorm expression
-// (crates/tritium-nn/src/ops/rmsnorm.rs:88-91), one rounding per operation.
-__device__ __forceinline__ void apply_norm(const DecodeParams& p, float inv, uint32_t col, float (&v)[8]) {
-  float w[8];
-  load8(p.norm_weight, TB_F32, col, w);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const float scale = p.norm_zero_centered ? __fadd_rn(1.0f, w[e]) : w[e];
-    v[e] = __fmul_rn(__fmul_rn(v[e], inv), scale);
-  }
-}
-
-// squared-ReLU gate for eight consecutive activations (see relu2_gate)
-__device__ __forceinline__ void apply_gate(const DecodeParams& p, size_t at, float (&v)[8]) {
-  float u[8];
-  load8(p.relu2_up, TB_F32, at, u);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = relu2_gate(v[e], u[e]);
-}
-
+// Bound by latency and by instruction fetch (the code runs once per launch, from a cold cache), so it is
+// kept short: every activation is loaded once and stays in registers up to kChunkPairs pairs, loops stay
+// rolled, packed arithmetic builds the entries.  The form before (eight activations per lane, loaded once
+// for the absmax and again for the codes, unrolled; byte arithmetic for the entries) took 8,700 clocks for
+// ten pairs, 4,650 of them in the straight-line quantisation.  2560 x 2560, one plane, 1 token: 7.8 -> 5.7 us
+// per launch; 13824 x 2560: 10.6 -> 8.1; 32 launches of a decoder's layers, norms and residuals included: 352 -> 267 us.
+//
+// Codes are staged with 128 added (u = x + 128).  Work item of the entry construction = one packed word w
+// of one (tile column, token, scale group): the 20 (B3) or 16 (D2) activations that meet the word's
+// digits are five (four) aligned 32-bit words of the staged codes, every one of them inside a single scale
+// group.  Their transformed values z = x_t - 3 x_(t-1) (B3; x_t for D2) are formed in 16-bit lanes as
+// z + 512 = u_t - 3 u_(t-1) + 768, which is positive, and split as 4*high + low into two table words.
+// Entries of words outside the scale group stay zero.
 template <int CODEC, bool DUAL, int M>
 __device__ __forceinline__ void build_tables(const DecodeParams& p, uint8_t* smem, uint32_t tid, uint32_t tp_seq) {
   constexpr int kNM = MmaCount<CODEC, DUAL>::value;
   constexpr uint32_t ncol = (DUAL ? 4 : 2) * M;
   constexpr bool B3 = CODEC == tbf::kB3;
-  constexpr uint32_t kDigits = B3 ? 5 : 4, kWords = B3 ? 13 : 16;   // digits per packed byte, packed words per tile-plane
+  constexpr uint32_t kDigits = B3 ? 5 : 4, kItems = B3 ? 14 : 16;   // digits per packed byte; words per tile-plane (B3: word 6 once per scale group)
   const uint32_t warp = tid >> 5, lane = tid & 31;
-  uint8_t* xq = smem + p.off_xq;                                                             // [kChunkPairs][kPairStride]
-  float* red = reinterpret_cast<float*>(smem + p.off_xq + kChunkPairs * kPairStride);       // [warp][4]
+  uint8_t* xq = smem + p.off_xq;
+  uint32_t* absmax_bits = reinterpret_cast<uint32_t*>(xq + kStageTokens);
+  float* inv_rms = reinterpret_cast<float*>(xq + kStageTokens) + 4;
+  float* scale_q = inv_rms + 4;
+  float* act_scale = reinterpret_cast<float*>(smem + p.off_actscale);
   uint32_t* ztab = reinterpret_cast<uint32_t*>(smem + p.off_z);
   int* cinit = reinterpret_cast<int*>(smem + p.off_cinit);
-  float* act_scale = reinterpret_cast<float*>(smem + p.off_actscale);
-  float scale_q[M], scale_out[M], inv_rms[M];
   const uint32_t pairs = p.tpr * M;
   const bool norm = p.norm_weight != nullptr;
-#pragma unroll
-  for (int t = 0; t < M; ++t) inv_rms[t] = 1.f;
   if (norm) {
     // RMSNorm prologue, in the reference's canonical order (crates/tritium-nn/src/ops/rmsnorm.rs:20-34,
     // crates/tritium-cuda/kernels/decode.cu:533-640): 256 slots, slot t folds x[t], x[t+256], ...
     // ascending; then the power-of-two tree part[t] += part[t+off].  The 256 consumer threads are
-    // the 256 slots.  The staging area is free until the quantise phase.
-    float* part = reinterpret_cast<float*>(xq);
-    float* inv_s = red + kWarps * 4;
-#pragma unroll
-    for (int t = 0; t < M; ++t) {
-      if (uint32_t(t) >= p.m) break;
+    // the 256 slots.
+    float* part = reinterpret_cast<float*>(xq + kStageSlots);
+    for (uint32_t i = tid * 32; i < p.k; i += kConsumerThreads * 32) {   // the weights come into L1 meanwhile
+      float unused;
+      asm volatile("ld.global.f32 %0, [%1];" : "=f"(unused) : "l"(p.norm_weight + i));
+    }
+#pragma unroll 1
+    for (uint32_t t = 0; t < p.m; ++t) {
       float acc = 0.f;
-      for (uint32_t i = tid; i < p.k; i += kConsumerThreads) {
-        const size_t at = size_t(t) * p.k + i;
-        const float v = p.x_dtype == TB_F32 ? static_cast<const float*>(p.x)[at]
-                                            : __bfloat162float(static_cast<const __nv_bfloat16*>(p.x)[at]);
-        acc = __fadd_rn(acc, __fmul_rn(v, v));
+#pragma unroll 1
+      for (uint32_t j = 0; j < p.tpr; j += 12) {
+        float v[12];
+#pragma unroll
+        for (uint32_t i = 0; i < 12; ++i) {
+          const size_t at = size_t(t) * p.k + (j + i) * 256 + tid;
+          v[i] = j + i >= p.tpr ? 0.f : p.x_dtype == TB_F32 ? static_cast<const float*>(p.x)[at] : __bfloat162float(static_cast<const __nv_bfloat16*>(p.x)[at]);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 12; ++i) acc = __fadd_rn(acc, __fmul_rn(v[i], v[i]));   // + 0 past the end: squares are never -0
       }
       part[tid] = acc;
       consumer_sync();
       if (tid < 128) part[tid] = __fadd_rn(part[tid], part[tid + 128]);
       consumer_sync();
-      if (tid < 64) part[tid] = __fadd_rn(part[tid], part[tid + 64]);
-      consumer_sync();
-      if (tid < 32) {
-        float v = __fadd_rn(part[tid], part[tid + 32]);
+      if (tid < 32) {   // slots t, t + 32, t + 64, t + 96: the tree's next two levels
+        float v = __fadd_rn(__fadd_rn(part[tid], part[tid + 64]), __fadd_rn(part[tid + 32], part[tid + 96]));
         for (int o = 16; o; o >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));   // lane t pairs with t + o
-        if (tid == 0) inv_s[t] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(v, float(p.k)), p.norm_eps)));
+        if (tid == 0) inv_rms[t] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(v, float(p.k)), p.norm_eps)));
       }
       consumer_sync();
     }
-#pragma unroll
-    for (int t = 0; t < M; ++t) inv_rms[t] = uint32_t(t) < p.m ? inv_s[t] : 1.f;
-    consumer_sync();   // the slots turn back into staging
   }
-  if (tid < kChunkPairs) *reinterpret_cast<uint4*>(xq + tid * kPairStride + 256) = make_uint4(0, 0, 0, 0);
-  if (p.x_dtype == TB_I8) {
+  const bool one_pass = pairs <= kChunkPairs, measure = p.x_dtype != TB_I8 && !p.act_absmax_in;
+  float v[kSteps][4];
+  // where the lane's four activations of step s are: pair, token, element
+  const auto locate = [&](uint32_t base, uint32_t s, uint32_t& pr, uint32_t& t, uint32_t& col) {
+    const uint32_t half = warp + s * kWarps;
+    pr = base + (half >> 1);
+    const uint32_t j = pr / M;
+    t = pr - j * M;
+    col = j * 256 + (half & 1) * 128 + lane * 4;
+    return pr < pairs && t < p.m;   // table entries of absent tokens are never read for an output
+  };
+  bool held = false;   // v holds the (only) chunk
+#pragma unroll 1
+  for (uint32_t pass = measure ? 0 : 1; pass < 2; ++pass) {
+#pragma unroll 1
+    for (uint32_t base = 0; base < pairs; base += kChunkPairs) {
+      uint32_t pr, t, col;
+      if (!held) {
+        // all loads of the pass, then the conversions
+        if (p.x_dtype == TB_F32) {
 #pragma unroll
-    for (int t = 0; t < M; ++t) { scale_q[t] = 1.f; scale_out[t] = uint32_t(t) < p.m ? p.act_scale_in[t] : 0.f; }
-  } else {
-    if (!p.act_absmax_in) {
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) load4_f32(static_cast<const float*>(p.x), size_t(t) * p.k + col, v[s]);
+        } else if (p.x_dtype == TB_BF16) {
+          uint2 raw[kSteps];
 #pragma unroll
-      for (int t = 0; t < M; ++t) {
-        float mx = 0.f;
-        for (uint32_t i = tid * 8; i < p.k && uint32_t(t) < p.m; i += kConsumerThreads * 8) {
-          float v[8];
-          load8(p.x, p.x_dtype, size_t(t) * p.k + i, v);
-          if (p.relu2_up) apply_gate(p, size_t(t) * p.k + i, v);
-          if (norm) apply_norm(p, inv_rms[t], i, v);
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) raw[s] = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.x) + size_t(t) * p.k + col);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[e]));
-        }
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) red[warp * 4 + t] = mx;
-      }
-      consumer_sync();
-    }
-    float* peer_gamma = red + kWarps * 4 + 4;   // [rank][token]
-    if (p.tp && !p.act_absmax_in) {
-      // Row shard: the row's absmax is the maximum over the ranks' slices.  CTA 0 pushes this
-      // slice's value, tagged with the round, into every peer's copy of the slot; every CTA then
-      // finds the peers' values in its own GPU's memory.  Two parities alternate, so a rank that
-      // is one round ahead cannot overwrite a value still being read.
-      const TbCommView& cv = p.comm_absmax;
-      const uint32_t par = tp_seq & 1u;
-      if (tid < cv.world && tid != cv.rank) {
-        if (blockIdx.x == 0) {
-          uint64_t* dst = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(cv.data[tid]) + kCommAbsmaxWords) + (par * kCommMaxWorld + cv.rank) * 4;
-          for (uint32_t t = 0; t < p.m; ++t) {
-            float mine = 0.f;
-            for (uint32_t w2 = 0; w2 < uint32_t(kWarps); ++w2) mine = fmaxf(mine, red[w2 * 4 + t]);
-            peer_store_u64(dst + t, (uint64_t(tp_seq) << 32) | __float_as_uint(mine));
+          for (uint32_t s = 0; s < kSteps; ++s) {
+            v[s][0] = __uint_as_float(raw[s].x << 16); v[s][1] = __uint_as_float(raw[s].x & 0xffff0000u);
+            v[s][2] = __uint_as_float(raw[s].y << 16); v[s][3] = __uint_as_float(raw[s].y & 0xffff0000u);
           }
-        }
-        const uint64_t* src = reinterpret_cast<const uint64_t*>(reinterpret_cast<const uint8_t*>(cv.data[cv.rank]) + kCommAbsmaxWords) + (par * kCommMaxWorld + tid) * 4;
-        const long long t0 = clock64();
-        for (uint32_t t = 0; t < p.m; ++t) {
-          float got = 0.f;
-          for (uint32_t i = 0;; ++i) {
-            const uint64_t v = peer_load_u64(src + t);
-            if (uint32_t(v >> 32) == tp_seq) { got = __uint_as_float(uint32_t(v)); break; }
-            if ((i & 63u) == 63u && clock64() - t0 > cv.wait_cycles) {
-              if (atomicOr(&p.status[TBS_FLAGS], TBF_WAIT_TIMEOUT) == 0) { p.status[TBS_INFO0] = tid; p.status[TBS_INFO1] = 600 + t; }
-              break;
+        } else {
+#pragma unroll
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) {
+              const char4 raw = *reinterpret_cast<const char4*>(static_cast<const int8_t*>(p.x) + size_t(t) * p.k + col);
+              v[s][0] = raw.x; v[s][1] = raw.y; v[s][2] = raw.z; v[s][3] = raw.w;
             }
-          }
-          peer_gamma[tid * 4 + t] = got;
         }
+        if (p.relu2_up) {   // squared-ReLU gate (see relu2_gate)
+          float u[kSteps][4];
+#pragma unroll
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) load4_f32(p.relu2_up, size_t(t) * p.k + col, u[s]);
+#pragma unroll
+          for (uint32_t s = 0; s < kSteps; ++s)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[s][e] = relu2_gate(v[s][e], u[s][e]);
+        }
+        if (norm) {
+          // y = (x * inv) * w (or (1 + w)): the reference's rmsnorm expression
+          // (crates/tritium-nn/src/ops/rmsnorm.rs:88-91), one rounding per operation
+          float w[kSteps][4];
+#pragma unroll
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) load4_f32(p.norm_weight, col, w[s]);
+#pragma unroll
+          for (uint32_t s = 0; s < kSteps; ++s)
+            if (locate(base, s, pr, t, col)) {
+              const float inv = inv_rms[t];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                v[s][e] = __fmul_rn(__fmul_rn(v[s][e], inv), p.norm_zero_centered ? __fadd_rn(1.0f, w[s][e]) : w[s][e]);
+            }
+        }
+        held = one_pass;
+      }
+      if (pass == 0) {
+#pragma unroll
+        for (uint32_t s = 0; s < kSteps; ++s)
+          if (locate(base, s, pr, t, col)) {
+            float mx = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) mx = fmaxf(mx, fabsf(v[s][e]));
+            const uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));   // non-negative floats order like their bits
+            if (lane == 0) atomicMax(absmax_bits + t, bits);
+          }
+        continue;
+      }
+      if (base == 0 && !measure) {   // scales from the caller
+        if (tid < p.m) {
+          const float gamma = p.x_dtype == TB_I8 ? 0.f : p.act_absmax_in[tid];
+          scale_q[tid] = p.x_dtype == TB_I8 ? 1.f : gamma > 0.f ? __fdiv_rn(127.0f, gamma) : 0.f;
+          act_scale[tid] = p.x_dtype == TB_I8 ? p.act_scale_in[tid] : __fdiv_rn(gamma, 127.0f);
+        }
+        consumer_sync();
+      }
+      // ---- codes, and the accumulator start values (see prepare_kernel)
+#pragma unroll
+      for (uint32_t s = 0; s < kSteps; ++s)
+        if (locate(base, s, pr, t, col)) {
+          const float sq = scale_q[t];
+          bool bad = false;
+          uint32_t q[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            bad |= !(fabsf(v[s][e]) <= FLT_MAX);
+            // adding 1.5 * 2^23 rounds to the nearest integer, ties to even, and leaves it in the low bits
+            q[e] = __float_as_uint(__fadd_rn(fminf(127.f, fmaxf(-128.f, __fmul_rn(v[s][e], sq))), 12582912.0f));
+          }
+          if (bad && atomicOr(&p.status[TBS_FLAGS], TBF_NONFINITE_ACT) == 0) {
+            p.status[TBS_INFO0] = t * p.k + col; p.status[TBS_INFO1] = 0x7fc00000u;
+          }
+          const uint32_t codes = prmt(prmt(q[0], q[1], 0x0040u), prmt(q[2], q[3], 0x0040u), 0x5410u);
+          const uint32_t half = warp + s * kWarps;
+          *reinterpret_cast<uint32_t*>(xq + (half >> 1) * kPairStride + (half & 1) * 128 + lane * 4) = codes ^ 0x80808080u;
+          // coefficients {1, -2, -1, -1, 2}[position mod 5] (B3) as bytes, four from the lane's first position on
+          const uint32_t coef = B3 ? __funnelshift_rc(0xfffffe01u, 0xfffe0102u, 8 * (((half & 1) * 128 + lane * 4) % 5)) : 0x01010101u;
+          const int sum = __reduce_add_sync(0xffffffffu, __dp4a(int(codes), int(coef), 0));
+          if (lane == 0) cinit[(t * p.tpr + pr / M) * 2 + (half & 1)] = -sum;
+        }
+      consumer_sync();
+      // ---- entries: item = (pair of the chunk, packed word and scale group)
+      const uint32_t lp = tid / kItems, item = tid - lp * kItems;
+      pr = base + lp;
+      const uint32_t j = pr / M;
+      t = pr - j * M;
+      if (lp < kChunkPairs && pr < pairs && t < p.m) {
+        const uint32_t w = B3 && item == 13 ? 6u : item, v2 = B3 ? (item >= 7 ? 1u : 0u) : w >> 3;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(xq + lp * kPairStride + 4 * kDigits * w);
+        uint32_t W[kDigits];
+#pragma unroll
+        for (uint32_t i = 0; i < kDigits; ++i) {
+          W[i] = src[i];   // trits 256..259 are the padding behind the pair
+          // word 6 of B3 holds trits 120..139: two words of group 0, three of group 1
+          if (B3 && w == 6 && (i < 2) != (v2 == 0)) W[i] = 0x80808080u;
+        }
+        uint32_t hi[kDigits], lo[kDigits];   // per digit, the packed word's four bytes
+        uint32_t even = 0, odd = 0;           // bytes 0, 2 and 1, 3 of the digit before, in 16-bit lanes
+#pragma unroll
+        for (uint32_t i = 0; i < kDigits; ++i) {
+          // activation kDigits * e + i meets digit i of byte e
+          const uint32_t ev = prmt(W[i >> 2], W[(2 * kDigits + i) >> 2], (i & 3u) | ((4u + ((2 * kDigits + i) & 3u)) << 8)) & 0x00ff00ffu;
+          const uint32_t od = prmt(W[(kDigits + i) >> 2], W[(3 * kDigits + i) >> 2], ((kDigits + i) & 3u) | ((4u + ((3 * kDigits + i) & 3u)) << 8)) & 0x00ff00ffu;
+          const bool first = !B3 || i == 0;
+          const uint32_t ze = first ? ev + 0x01800180u : ev + 0x03000300u - 3u * even, zo = first ? od + 0x01800180u : od + 0x03000300u - 3u * odd;
+          even = ev; odd = od;
+          hi[i] = prmt(ze >> 2, zo >> 2, 0x6240u) ^ 0x80808080u;
+          lo[i] = prmt(ze, zo, 0x6240u) & 0x03030303u;
+        }
+        const uint32_t slot = w >> 2, c = w & 3, col0 = (DUAL ? v2 * 2 * M : 0) + 2 * t;
+        const uint32_t mma = first_mma_of<CODEC, DUAL>(slot, v2);
+        uint2* at = reinterpret_cast<uint2*>(ztab) + ((j * kNM + mma) * ncol + col0) * 4;
+        if (B3 && slot == 3) {
+          // byte e of word 12 belongs to lane column e: operand quad 0 = digits 0..3, quad 1 byte 0 = digit 4
+#pragma unroll
+          for (uint32_t part = 0; part < 2; ++part) {
+            const uint32_t* d = part ? lo : hi;
+            const uint32_t a01 = prmt(d[0], d[1], 0x5140u), a23 = prmt(d[2], d[3], 0x5140u), b01 = prmt(d[0], d[1], 0x7362u), b23 = prmt(d[2], d[3], 0x7362u);
+            at[part * 4 + 0] = make_uint2(prmt(a01, a23, 0x5410u), d[4] & 0xffu);
+            at[part * 4 + 1] = make_uint2(prmt(a01, a23, 0x7632u), (d[4] >> 8) & 0xffu);
+            at[part * 4 + 2] = make_uint2(prmt(b01, b23, 0x5410u), (d[4] >> 16) & 0xffu);
+            at[part * 4 + 3] = make_uint2(prmt(b01, b23, 0x7632u), d[4] >> 24);
+          }
+        } else {
+          // digits 2i and 2i + 1 are the two operand quads of MMA `mma` + i; low parts: the next column
+#pragma unroll
+          for (uint32_t i = 0; i < (kDigits + 1) / 2; ++i) {
+            at[i * ncol * 4 + c] = make_uint2(hi[2 * i], 2 * i + 1 < kDigits ? hi[2 * i + 1 < kDigits ? 2 * i + 1 : 0] : 0u);
+            at[i * ncol * 4 + 4 + c] = make_uint2(lo[2 * i], 2 * i + 1 < kDigits ? lo[2 * i + 1 < kDigits ? 2 * i + 1 : 0] : 0u);
+          }
+        }
+      }
+      if (!one_pass) consumer_sync();   // the staging is written again
+    }
+    if (pass == 0) {
+      consumer_sync();
+      float* peer_gamma = reinterpret_cast<float*>(xq + kStagePeers);   // [rank][token]
+      if (p.tp) {
+        // Row shard: the row's absmax is the maximum over the ranks' slices.  CTA 0 pushes this
+        // slice's value, tagged with the round, into every peer's copy of the slot; every CTA then
+        // finds the peers' values in its own GPU's memory.  Two parities alternate, so a rank that
+        // is one round ahead cannot overwrite a value still being read.
+        const TbCommView& cv = p.comm_absmax;
+        const uint32_t par = tp_seq & 1u;
+        if (tid < cv.world && tid != cv.rank) {
+          if (blockIdx.x == 0) {
+            uint64_t* dst = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(cv.data[tid]) + kCommAbsmaxWords) + (par * kCommMaxWorld + cv.rank) * 4;
+            for (uint32_t t = 0; t < p.m; ++t)
+              peer_store_u64(dst + t, (uint64_t(tp_seq) << 32) | absmax_bits[t]);
+          }
+          const uint64_t* src = reinterpret_cast<const uint64_t*>(reinterpret_cast<const uint8_t*>(cv.data[cv.rank]) + kCommAbsmaxWords) + (par * kCommMaxWorld + tid) * 4;
+          const long long t0 = clock64();
+          for (uint32_t t = 0; t < p.m; ++t) {
+            float got = 0.f;
+            for (uint32_t i = 0;; ++i) {
+              const uint64_t v = peer_load_u64(src + t);
+              if (uint32_t(v >> 32) == tp_seq) { got = __uint_as_float(uint32_t(v)); break; }
+              if ((i & 63u) == 63u && clock64() - t0 > cv.wait_cycles) {
+                if (atomicOr(&p.status[TBS_FLAGS], TBF_WAIT_TIMEOUT) == 0) { p.status[TBS_INFO0] = tid; p.status[TBS_INFO1] = 600 + t; }
+                break;
+              }
+            }
+            peer_gamma[tid * 4 + t] = got;
+          }
+        }
+        consumer_sync();
+      }
+      if (tid < p.m) {
+        float gamma = __uint_as_float(absmax_bits[tid]);
+        if (p.tp)
+          for (uint32_t r = 0; r < p.comm_absmax.world; ++r)
+            if (r != p.comm_absmax.rank) gamma = fmaxf(gamma, peer_gamma[r * 4 + tid]);
+        scale_q[tid] = gamma > 0.f ? __fdiv_rn(127.0f, gamma) : 0.f;
+        act_scale[tid] = __fdiv_rn(gamma, 127.0f);
       }
       consumer_sync();
     }
-#pragma unroll
-    for (int t = 0; t < M; ++t) {
-      float gamma = 0.f;
-      if (p.act_absmax_in) gamma = uint32_t(t) < p.m ? p.act_absmax_in[t] : 0.f;   // absmax over the full (unsharded) row, supplied by the caller
-      else {
-        for (uint32_t w2 = 0; w2 < uint32_t(kWarps); ++w2) gamma = fmaxf(gamma, red[w2 * 4 + t]);
-        if (p.tp && uint32_t(t) < p.m)
-          for (uint32_t r = 0; r < p.comm_absmax.world; ++r)
-            if (r != p.comm_absmax.rank) gamma = fmaxf(gamma, peer_gamma[r * 4 + t]);
-      }
-      scale_q[t] = gamma > 0.f ? __fdiv_rn(127.0f, gamma) : 0.f;
-      scale_out[t] = __fdiv_rn(gamma, 127.0f);
-    }
-  }
-  for (uint32_t base = 0; base < pairs; base += kChunkPairs) {
-    const uint32_t chunk = min(kChunkPairs, pairs - base);
-    // ---- quantise: a warp takes whole pairs (lane = eight consecutive activations), and adds up
-    // the accumulator start values of the pair's two scale groups on the way
-#pragma unroll
-    for (uint32_t r = 0; r < kChunkPairs / kWarps; ++r) {
-      const uint32_t lp = warp + r * kWarps;
-      if (lp >= chunk) continue;
-      const uint32_t pr = base + lp, j = pr / M, t = pr - j * M;
-      if (t >= p.m) continue;   // table entries of absent tokens are never read for an output
-      float v[8];
-      load8(p.x, p.x_dtype, size_t(t) * p.k + j * 256 + lane * 8, v);
-      float sq = scale_q[0], inv = inv_rms[0];
-#pragma unroll
-      for (int tt = 1; tt < M; ++tt) { sq = t == uint32_t(tt) ? scale_q[tt] : sq; inv = t == uint32_t(tt) ? inv_rms[tt] : inv; }
-      if (p.relu2_up) apply_gate(p, size_t(t) * p.k + j * 256 + lane * 8, v);
-      if (norm) apply_norm(p, inv, j * 256 + lane * 8, v);
-      int q[8];
-      bool bad = false;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        bad |= !(fabsf(v[e]) <= FLT_MAX);
-        q[e] = p.x_dtype == TB_I8 ? int(v[e]) : int(fminf(127.f, fmaxf(-128.f, rintf(__fmul_rn(v[e], sq)))));
-      }
-      if (bad && atomicOr(&p.status[TBS_FLAGS], TBF_NONFINITE_ACT) == 0) {
-        p.status[TBS_INFO0] = t * p.k + j * 256 + lane * 8; p.status[TBS_INFO1] = 0x7fc00000u;
-      }
-      uint2 packed;
-      packed.x = uint32_t(q[0] & 0xff) | (uint32_t(q[1] & 0xff) << 8) | (uint32_t(q[2] & 0xff) << 16) | (uint32_t(q[3] & 0xff) << 24);
-      packed.y = uint32_t(q[4] & 0xff) | (uint32_t(q[5] & 0xff) << 8) | (uint32_t(q[6] & 0xff) << 16) | (uint32_t(q[7] & 0xff) << 24);
-      reinterpret_cast<uint2*>(xq + lp * kPairStride)[lane] = packed;
-      // accumulator start values (see prepare_kernel): lanes 0..15 hold scale group 0, 16..31 group 1
-      int sum = 0;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        int coef = 1;
-        if (B3) { const int d = int(lane * 8 + e) % 5; coef = d == 0 ? 1 : d == 1 ? -2 : d == 4 ? 2 : -1; }
-        sum += q[e] * coef;
-      }
-      for (int o = 8; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if ((lane & 15) == 0) cinit[(t * p.tpr + j) * 2 + (lane >> 4)] = -sum;
-    }
-    consumer_sync();
-    // ---- entries: item = (pair of the chunk, scale group, packed word position)
-    for (uint32_t item = tid; item < chunk * 2 * kWords; item += kConsumerThreads) {
-      const uint32_t lp = item / (2 * kWords), rem = item - lp * (2 * kWords), v = rem / kWords, w = rem - v * kWords;
-      const uint32_t pr = base + lp, j = pr / M, t = pr - j * M;
-      if (t >= p.m) continue;
-      const uint32_t slot = w >> 2, c = w & 3;
-      const bool bytewise = B3 && slot == 3;
-      if (!DUAL && mma_of<CODEC, false>(slot, 0, v) < 0) continue;   // no MMA reads this word for this scale group
-      // the activations that meet the digits of packed word w: words of four, each inside one scale group
-      const uint32_t t0 = 4 * kDigits * w;
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(xq + lp * kPairStride + t0);
-      int a[4 * 5];
-#pragma unroll
-      for (uint32_t kw = 0; kw < kDigits; ++kw) {
-        const uint32_t word = (((t0 + 4 * kw) >> 7) == v) ? src[kw] : 0u;   // trits 256..259 read the zero padding
-#pragma unroll
-        for (int b = 0; b < 4; ++b) a[4 * kw + b] = sbyte(word, b);
-      }
-      // z of (byte e, digit i) and its parts
-      uint32_t hi[5][4], lo[5][4];   // [digit][byte]
-#pragma unroll
-      for (uint32_t e = 0; e < 4; ++e) {
-#pragma unroll
-        for (uint32_t i = 0; i < kDigits; ++i) {
-          const int cur = a[kDigits * e + i];
-          const int z = (B3 && i > 0) ? cur - 3 * a[kDigits * e + i - 1] : cur;
-          hi[i][e] = uint32_t(z >> 2) & 0xffu;
-          lo[i][e] = uint32_t(z) & 3u;
-        }
-      }
-      const uint32_t col0 = (DUAL ? v * 2 * M : 0) + 2 * t;
-      if (bytewise) {
-        // byte e of word 12 belongs to lane column e: operand quad 0 = digits 0..3, quad 1 byte 0 = digit 4
-        const uint32_t mma = uint32_t(mma_of<CODEC, DUAL>(3, 0, v));
-#pragma unroll
-        for (uint32_t e = 0; e < 4; ++e) {
-          uint32_t* at = ztab + (((j * kNM + mma) * ncol + col0) * 4 + e) * 2;
-          at[0] = hi[0][e] | (hi[1][e] << 8) | (hi[2][e] << 16) | (hi[3][e] << 24); at[1] = hi[4][e];
-          at[8] = lo[0][e] | (lo[1][e] << 8) | (lo[2][e] << 16) | (lo[3][e] << 24); at[9] = lo[4][e];
-        }
-      } else {
-#pragma unroll
-        for (uint32_t i = 0; i < kDigits; ++i) {
-          // digit i: MMA of (slot, digit pair i/2), operand quad i%2; bytes e = 0..3
-          const uint32_t mma = uint32_t(mma_of<CODEC, DUAL>(slot, i >> 1, v));
-          uint32_t* at = ztab + (((j * kNM + mma) * ncol + col0) * 4 + c) * 2 + (i & 1);
-          at[0] = hi[i][0] | (hi[i][1] << 8) | (hi[i][2] << 16) | (hi[i][3] << 24);
-          at[8] = lo[i][0] | (lo[i][1] << 8) | (lo[i][2] << 16) | (lo[i][3] << 24);   // low part: the next column
-          if (B3 && i == 4) { at[1] = 0u; at[9] = 0u; }                                 // the fifth digit has no partner
-        }
-      }
-    }
-    consumer_sync();
-  }
-  if (tid < uint32_t(M)) {
-    float so = scale_out[0];
-#pragma unroll
-    for (int tt = 1; tt < M; ++tt) so = tid == uint32_t(tt) ? scale_out[tt] : so;
-    act_scale[tid] = so;
   }
 }
 
@@ -763,7 +780,10 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   constexpr int YN = kPlaneSets ? 1 : SETS;       // partial sums a lane keeps for each of its two rows
   constexpr uint32_t kSliceFloats = YN * 16 * NC;   // one consumer warp's partial sums of a row block
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], table_bar, part_full[kPartBufs], part_empty[kPartBufs];
+  // barriers: per ring slot "full" and "empty", per partial-sum buffer "full" and "empty", the tables
+  __shared__ uint64_t bars[2 * kMaxStages + 2 * kPartBufs + 1];
+  uint64_t *full_bar = bars, *empty_bar = bars + kMaxStages, *part_full = empty_bar + kMaxStages, *part_empty = part_full + kPartBufs;
+  uint64_t& table_bar = part_empty[kPartBufs];
   __shared__ uint32_t abort_flag, tp_round;
   __shared__ TbLayerDesc layer_desc[kMaxGroupLayers];
 
@@ -775,13 +795,12 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   float* part = reinterpret_cast<float*>(smem + p.off_part);
   const float* act_scale = reinterpret_cast<const float*>(smem + p.off_actscale);
 
-  if (tid == 0) {
-    abort_flag = 0;
-    for (uint32_t s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kWarps); }
-    mbar_init(&table_bar, 1);
-    for (int b = 0; b < kPartBufs; ++b) { mbar_init(&part_full[b], kWarps); mbar_init(&part_empty[b], 1); }
+  if (tid < 2 * kMaxStages + 2 * kPartBufs + 1) {   // the consumer warps arrive on "empty" ring slots and "full" buffers
+    const bool by_consumers = (tid >= kMaxStages && tid < 2 * kMaxStages + kPartBufs);
+    mbar_init(&bars[tid], by_consumers ? kWarps : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (tid == 0) abort_flag = 0;
   for (uint32_t l = tid; l < p.layer_count; l += kThreads) {
     if (p.layers) { layer_desc[l].payload = p.layers[l].payload; layer_desc[l].scales = p.layers[l].scales; }
     else { layer_desc[l].payload = p.payload; layer_desc[l].scales = p.scales; }
@@ -948,6 +967,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
 
   // -------------------------------------------------- consumers: activation tables
   if (p.fused) {
+    clear_tables(p, smem, tid);
+    consumer_sync();
     // x may be the previous kernel's output: wait for it (the weight stream is already running)
     if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.tp) {
@@ -1268,10 +1289,13 @@ bool tb_decode_supported(const tb_weights* w, uint32_t m, int max_smem, size_t* 
 size_t tb_decode_scratch_bytes(const tb_weights* w, uint32_t m) { return table_layout(w, m).total; }
 
 bool tb_decode_builds_tables(const tb_weights* w, uint32_t m, const void* x) {
-  // (tile column, token) pairs every CTA would have to quantise and lay out; measured on B200: up
-  // to about a dozen pairs the single launch wins, beyond that the separate kernel
-  const uint32_t pairs = uint32_t(w->k / 256) * layout_tokens(m);
-  return pairs <= 12 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  // Every CTA quantises and lays out all (tile column, token) pairs.  Measured on B200, us per call in a graph,
+  // in the kernel / preparation kernel in front: one token, 20 pairs 30.7 / 30.8 (34816 x 5120) and 11.2 / 10.9
+  // (5120 x 5120), 27 pairs 9.2 / 9.7 (2560 x 6912), 68 pairs 26.5 / 21.8 (5120 x 17408); four tokens, 40 pairs
+  // 15.2 / 12.1, 80 pairs 18.1 / 12.1.  Level at 20 pairs, where the second launch costs the host 2 us besides; a
+  // four-token table has twice the entries per pair and goes by one pass of the builder.
+  const uint32_t mk = layout_tokens(m), pairs = uint32_t(w->k / 256) * mk;
+  return pairs <= (use_dual(mk) ? 32u : 16u) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
 }
 
 cudaError_t tb_launch_prepare(const DecodeArgs& a, cudaStream_t stream) {
