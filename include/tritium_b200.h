@@ -102,6 +102,13 @@ void tb_backend_free(tb_backend* backend);
 /* TernaryBackend::capabilities (crates/tritium-spec/src/lib.rs:166-185). */
 tb_status tb_backend_caps(const tb_backend* backend, tb_caps* out);
 tb_status tb_backend_synchronize(tb_backend* backend);
+/* Pinned host memory for outputs of the host-pointer calls.  A call whose whole output lies in such a
+ * buffer copies the result straight into it, where other outputs pass through a bounce buffer; the one
+ * difference in behaviour is that such an output may have been written when the call fails.  No
+ * counterpart in the reference (its outputs are Vec<f32>).  tb_host_free takes NULL and buffers of a
+ * backend that was freed. */
+tb_status tb_host_alloc(tb_backend* backend, size_t bytes, void** out);
+void tb_host_free(void* buffer);
 
 /* ------------------------------------------------------------------ weights
  * TernaryBackend::upload_weights for TernaryFormat::Tq2_0 (crates/tritium-spec/src/lib.rs:186-199,

@@ -659,3 +659,32 @@ def test_exact_kernel_leaves_out_zero_trits_of_nonfinite_activations(backend, ba
     same[token, reached] = False
     assert np.array_equal(got.view(np.uint32)[same], want.view(np.uint32)[same])
     assert not np.isfinite(got[~same]).any()
+
+
+@pytest.mark.parametrize("m", [1, 40])
+def test_host_outputs_keep_their_memory(m):
+    """Outputs of host calls lie in pinned buffers that are used again once the array is gone: arrays that are kept
+    hold their values through later calls and through the end of the backend, and a failing call gives none away."""
+    from tritium_b200 import B200Backend
+    b = B200Backend(0)
+    n, k = 2304, 512
+    prod, orac = uniform_pair(n, k, 2, seed=5)
+    resident = b.upload_salt_v2(prod, SaltV2Codec.B3)
+    xs = [make_activations(m, k, seed=i, bf16=True) for i in range(4)]
+    kept = [b.salt_v2_forward_fast(resident, x, m).output for x in xs]
+    for x in xs:
+        b.salt_v2_forward_fast(resident, x, m)          # dropped at once
+        b.linear_forward_a8(resident, x, m)
+    with pytest.raises(errors.InvalidInput):
+        b.salt_v2_forward_exact(resident, np.full((m, k), np.nan, np.float32), m)
+    exact = b.salt_v2_forward_exact(resident, xs[0], m).output
+    tail = kept[1][:, 7:]                               # a view alone keeps the buffer
+    want = [orc.matmul(orac, x) for x in xs]
+    del kept[1]
+    b.salt_v2_forward_fast(resident, xs[3], m)
+    resident.free()
+    b.close()
+    assert rel_l2(tail, want[1][:, 7:]) <= 1e-5
+    for got, i in zip(kept, (0, 2, 3)):
+        assert rel_l2(got, want[i]) <= 1e-5 and got.flags.writeable and got.shape == (m, n)
+    assert np.array_equal(exact.view(np.uint32), want[0].view(np.uint32))

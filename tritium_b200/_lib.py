@@ -29,7 +29,7 @@ EXPORTS = [
     "tb_fmt_resident_sizes", "tb_fmt_resident_build", "tb_fmt_package_write", "tb_fmt_tq2_pack_rows",
     "tb_fmt_quantize_act_int8", "tb_linear_forward_a8_static", "tb_backend_inject_wait_timeout",
     "tb_salt_v2_upload_reader", "tb_fmt_package_write_multi", "tb_fmt_package_extract", "tb_last_shape_mismatch", "tb_salt_v1_upload", "tb_tq1_upload",
-    "tb_fmt_device_layout", "tb_gemm_registers_check",
+    "tb_fmt_device_layout", "tb_gemm_registers_check", "tb_host_alloc", "tb_host_free",
 ]
 
 
@@ -131,6 +131,8 @@ _SIGNATURES = {
     "tb_backend_free": (None, [_P]),
     "tb_backend_caps": (_ST, [_P, _P]),
     "tb_backend_synchronize": (_ST, [_P]),
+    "tb_host_alloc": (_ST, [_P, _SZ, _P]),
+    "tb_host_free": (None, [_P]),
     "tb_tq2_upload": (_ST, [_P, _P, _SZ, _U32, _U32, _P]),
     "tb_tq1_upload": (_ST, [_P, _P, _SZ, _U32, _U32, _P]),
     "tb_salt_v1_upload": (_ST, [_P, _P, _SZ, _U32, _U32, _U32, _P]),

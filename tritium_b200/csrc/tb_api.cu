@@ -1,9 +1,12 @@
 // C ABI of the B200 backend: handles, uploads, forward entry points, stack driver, host format
 // helpers.  Host logic only; kernels live in kernels_*.cu.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -68,7 +71,55 @@ tb_status use_device(const tb_backend* b) {
   return TB_OK;
 }
 
+// Output buffers that tb_host_alloc handed out: start -> bytes.  A call whose output lies in one of them
+// copies straight into it.
+std::mutex g_host_lock;
+std::map<uintptr_t, size_t> g_host_buffers;
+bool host_buffer_holds(const void* p, size_t bytes) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  std::lock_guard<std::mutex> hold(g_host_lock);
+  auto it = g_host_buffers.upper_bound(a);
+  if (it == g_host_buffers.begin()) return false;
+  --it;
+  return a - it->first <= it->second && bytes <= it->second - (a - it->first);
+}
+// Pinning memory must not break a stream capture that runs in another thread.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 }  // namespace
+
+extern "C" tb_status tb_host_alloc(tb_backend* b, size_t bytes, void** out) {
+  clear_error();
+  if (!b || !out) return tb_fail(TB_NULL_ARG, "null argument");
+  *out = nullptr;
+  if (!bytes) return tb_fail(TB_INVALID_INPUT, "a host buffer has at least one byte");
+  if (tb_status s = use_device(b)) return s;
+  const RelaxedCapture relaxed;
+  void* p = nullptr;
+  TB_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocPortable), "allocate host buffer");
+  try {
+    std::lock_guard<std::mutex> hold(g_host_lock);
+    g_host_buffers[reinterpret_cast<uintptr_t>(p)] = bytes;
+  } catch (...) {
+    cudaFreeHost(p);
+    return tb_fail(TB_OUT_OF_MEMORY, "host allocation failed");
+  }
+  *out = p;
+  return TB_OK;
+}
+
+extern "C" void tb_host_free(void* p) {
+  {
+    std::lock_guard<std::mutex> hold(g_host_lock);
+    if (!g_host_buffers.erase(reinterpret_cast<uintptr_t>(p))) return;
+  }
+  const RelaxedCapture relaxed;
+  cudaFreeHost(p);
+}
 
 extern "C" tb_status tb_backend_create(int ordinal, tb_backend** out) {
   clear_error();
@@ -555,8 +606,10 @@ tb_status forward_host(tb_backend* b, const tb_weights* w, const void* x, tb_dty
   uint8_t* aux = static_cast<uint8_t*>(b->d_aux);
   // Activations and outputs travel through one pinned bounce buffer, so that both copies are truly
   // asynchronous and the call needs a single stream synchronisation: [x | y].
+  // An output in a buffer of tb_host_alloc is pinned itself and is copied to directly.
   const size_t x_off = 0, y_off = (xb + 255) / 256 * 256;
-  if (tb_status s = ensure(&b->h_pin, &b->h_pin_cap, y_off + yb, true)) return s;
+  const bool direct = host_buffer_holds(y, yb);
+  if (tb_status s = ensure(&b->h_pin, &b->h_pin_cap, y_off + (direct ? 0 : yb), true)) return s;
   uint8_t* pin = static_cast<uint8_t*>(b->h_pin);
   std::memcpy(pin + x_off, x, xb);
   TB_CUDA(cudaMemcpyAsync(b->d_x, pin + x_off, xb, cudaMemcpyHostToDevice, b->stream), "copy activations to device");
@@ -568,11 +621,11 @@ tb_status forward_host(tb_backend* b, const tb_weights* w, const void* x, tb_dty
   if (tb_status s = forward_dev(b, w, a, b->stream, receipt)) return s;
   // the device status word (bounded waits, finite checks) comes back with the output; the
   // caller's buffers are written only when it is clean
-  TB_CUDA(cudaMemcpyAsync(pin + y_off, b->d_y, yb, cudaMemcpyDeviceToHost, b->stream), "copy output to host");
+  TB_CUDA(cudaMemcpyAsync(direct ? y : pin + y_off, b->d_y, yb, cudaMemcpyDeviceToHost, b->stream), "copy output to host");
   TB_CUDA(cudaMemcpyAsync(b->h_status, b->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream), "read status");
   TB_CUDA(cudaStreamSynchronize(b->stream), "synchronize stream");
   if (b->h_status[TBS_FLAGS]) return tb_backend_check(b, b->stream);   // reports and clears
-  std::memcpy(y, pin + y_off, yb);
+  if (!direct) std::memcpy(y, pin + y_off, yb);
   if (dump_b) {
     TB_CUDA(cudaMemcpyAsync(acc_dump, aux, dump_b, cudaMemcpyDeviceToHost, b->stream), "copy accumulators to host");
     TB_CUDA(cudaStreamSynchronize(b->stream), "synchronize stream");
@@ -581,14 +634,21 @@ tb_status forward_host(tb_backend* b, const tb_weights* w, const void* x, tb_dty
 }
 
 tb_status preflight_finite(const float* x, size_t count) {
-  for (size_t i = 0; i < count; ++i)
-    if (!std::isfinite(x[i])) {
-      uint32_t bits;
-      std::memcpy(&bits, &x[i], 4);
-      char msg[96];
-      std::snprintf(msg, sizeof msg, "SALT V2 activation %zu is non-finite (%#010x)", i, bits);
-      return tb_fail(TB_INVALID_INPUT, msg);
-    }
+  constexpr size_t kBlock = 1024;   // no exit inside a block, so that the loop becomes vector code
+  for (size_t base = 0; base < count; base += kBlock) {
+    const size_t end = std::min(count, base + kBlock);
+    uint32_t bad = 0;
+    for (size_t i = base; i < end; ++i) bad |= uint32_t(!(std::fabs(x[i]) <= FLT_MAX));
+    if (!bad) continue;
+    for (size_t i = base; i < end; ++i)
+      if (!std::isfinite(x[i])) {
+        uint32_t bits;
+        std::memcpy(&bits, &x[i], 4);
+        char msg[96];
+        std::snprintf(msg, sizeof msg, "SALT V2 activation %zu is non-finite (%#010x)", i, bits);
+        return tb_fail(TB_INVALID_INPUT, msg);
+      }
+  }
   return TB_OK;
 }
 
@@ -1004,21 +1064,22 @@ extern "C" tb_status tb_stack_forward_host(tb_stack* st, const void* x, tb_dtype
   for (const tb_weights* w : st->layers) yb += size_t(m) * w->n * 2;
   const size_t y_off = (xb + 255) / 256 * 256;
   if (tb_status s = ensure(&b->d_x, &b->d_x_cap, xb)) return s;
-  if (tb_status s = ensure(&b->h_pin, &b->h_pin_cap, y_off + yb, true)) return s;
+  const bool direct = host_buffer_holds(y_bf16, yb);
+  if (tb_status s = ensure(&b->h_pin, &b->h_pin_cap, y_off + (direct ? 0 : yb), true)) return s;
   uint8_t* pin = static_cast<uint8_t*>(b->h_pin);
   std::memcpy(pin, x, xb);
   TB_CUDA(cudaMemcpyAsync(b->d_x, pin, xb, cudaMemcpyHostToDevice, b->stream), "copy activations to device");
   if (tb_status s = tb_stack_forward_dev(st, b->d_x, xd, m, nullptr, TB_BF16, flags, b->stream)) return s;
-  size_t off = y_off;
+  uint8_t* out = direct ? static_cast<uint8_t*>(y_bf16) : pin + y_off;
   for (const StackGroup& g : st->groups) {
     const size_t bytes = g.count * size_t(m) * st->layers[g.first]->n * 2;
-    TB_CUDA(cudaMemcpyAsync(pin + off, g.y, bytes, cudaMemcpyDeviceToHost, b->stream), "copy group outputs to host");
-    off += bytes;
+    TB_CUDA(cudaMemcpyAsync(out, g.y, bytes, cudaMemcpyDeviceToHost, b->stream), "copy group outputs to host");
+    out += bytes;
   }
   TB_CUDA(cudaMemcpyAsync(b->h_status, b->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream), "read status");
   TB_CUDA(cudaStreamSynchronize(b->stream), "synchronize stream");
   if (b->h_status[TBS_FLAGS]) return tb_backend_check(b, b->stream);
-  std::memcpy(y_bf16, pin + y_off, yb);
+  if (!direct) std::memcpy(y_bf16, pin + y_off, yb);
   return TB_OK;
 }
 
