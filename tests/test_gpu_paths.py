@@ -527,6 +527,35 @@ def test_wide_token_tiles_at_their_edges(backend, codec, k, planes):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
+@pytest.mark.parametrize("k,planes", [(2560, 1), (3072, 1), (3328, 2), (2304, 3)])
+def test_tiles_of_128_tokens_that_split_k(backend, codec, k, planes):
+    """Three row tiles (the last one ragged) whose K is shared by up to eight CTAs, evenly or not, and one that is
+    just not worth it (2560, 1 plane): a half tile and one more token, a full tile and one more, three tiles.
+    Sampled rows against the oracle; the parts are added in a fixed order, so a second run gives the same bits."""
+    import torch
+    from gpu_common import oracle_rows, product_only, sample_rows
+    n = 300
+    prod = product_only(n, k, planes, seed=k)
+    rows = sample_rows(n)
+    orac, resident = oracle_rows(prod, rows), backend.upload_salt_v2(prod, codec)
+    backend.reserve(resident, 300)
+    for m in (65, 128, 129, 300):
+        x = make_activations(m, k, seed=m, bf16=True)
+        x_dev = torch.from_numpy(x).cuda().to(torch.bfloat16)
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        dump = torch.zeros(m, n, k // 128, planes, dtype=torch.int32, device="cuda")
+        backend.forward_dev(resident, x_dev, y, a8=True, acc_dump=dump)
+        torch.cuda.synchronize()
+        backend.check()
+        want, want_dump, _ = orc.a8_linear(orac, x, dump=True)
+        at = torch.from_numpy(rows).cuda()
+        assert np.array_equal(dump[:, at].cpu().numpy(), want_dump[..., :planes]), m
+        assert rel_l2(y[:, at].cpu().numpy(), want) <= 1e-5, m
+        outputs_follow_without_the_dump(backend, resident, x_dev, y)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m", [24, 200])
 @pytest.mark.parametrize("dtype", ["bf16", "f32", "int8"])
 def test_unaligned_activations_in_front_of_the_tensor_cores(backend, m, dtype):

@@ -63,6 +63,7 @@ template <int TT> struct Tile {
   static constexpr int kThreads = 32 * (kFirstExpandWarp + kGroupWarps * kExpGroups);
   // an accumulator holds one slab of a 256-token tile, the two slabs of a tile-plane of a smaller one
   static constexpr bool kSingle = TT == 256;
+  static constexpr bool kMaySplit = !kSingle;   // a 256-token tile's sums are too many to pass through memory
   static constexpr int kAccBufs = TT >= 128 ? 2 : 4;
   static constexpr uint32_t kAccCols = kSingle ? TT : TT * 2;
   // "Weights are in shared memory" barriers and their counterparts.  256 tokens: one per slab, so that
@@ -106,7 +107,7 @@ struct PrefillParams {
   uint32_t m, m_pad, n, k, tpr, y_dtype;
   uint32_t n_tiles, m_tiles;
   // Split K: `splits` CTAs share an output tile, each walks a range of tile columns and leaves its
-  // fp32 running sums in `partial` [split][m_pad][n]; the last of them to finish (a counter per
+  // fp32 running sums in `partial` [split][m_pad][n] (m_pad: whole token tiles); the last of them to finish (a counter per
   // tile) adds the parts in split order and finishes the outputs.  splits == 1: none of this.
   uint32_t splits;
   float* partial; uint32_t* tile_counters;
@@ -705,6 +706,7 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(scale_slot), "l"(reinterpret_cast<const uint32_t*>(p.scales) + tp) : "memory");
     };
     const uint32_t tok0 = mt * TT + colhalf * kCW;
+    const bool live = T::kSingle || tok0 < p.m;   // else the drain would only take issue slots from the expanders
     const uint32_t row_tp = min(n, p.n - 1) * (p.tpr * PLANES);
     uint32_t tp = row_tp + j0 * PLANES;
     const uint32_t tp_end = row_tp + j1 * PLANES;
@@ -715,6 +717,10 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
       uint32_t sc;
       asm volatile("ld.shared.b32 %0, [%1];" : "=r"(sc) : "r"(scale_slot) : "memory");
       if (tp + 1 < tp_end) fetch_scale(tp + 1);
+      if (!live) {   // nothing but padding tokens in this half: hand the accumulator back
+        mbar_wait(full0 + 8 * buf, parity, wctx, 306);
+        if (lane == 0) mbar_arrive(empty0 + 8 * buf);
+      } else
 #pragma unroll
       for (uint32_t gsel = 0; gsel < 2; ++gsel) {
         const float sv = __half2float(__ushort_as_half(uint16_t(gsel ? sc >> 16 : sc & 0xffffu)));
@@ -758,8 +764,8 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
       waited = true;
     }
     const float rs = p.row_scale ? p.row_scale[min(n, p.n - 1)] : 1.0f;
-    if (n < p.n) {
-      if (p.splits > 1) {
+    if (live && n < p.n) {
+      if (T::kMaySplit && p.splits > 1) {
         float* part = p.partial + (size_t(sp) * p.m_pad + tok0) * p.n + n;   // padding tokens too: the scratch holds m_pad rows
 #pragma unroll
         for (uint32_t i = 0; i < kCW; ++i, part += p.n) *part = y[i];
@@ -770,7 +776,7 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
     }
 #pragma unroll
     for (uint32_t i = 0; i < kCW; ++i) y[i] = 0.f;
-    if (p.splits > 1) {
+    if (T::kMaySplit && p.splits > 1) {
       // Split K: count this split in; whoever completes the count adds the splits' sums in split
       // order (every run gives the same bits) and finishes the tile's outputs.
       __threadfence();
@@ -783,19 +789,26 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
       named_sync(kBarEpilogue, 32 * kEpilogueWarps);
       if (*combine_flag && n < p.n) {
         __threadfence();
+        // Each round of loads is one latency of L2, so as many as the registers hold (16 at a time: 2560 x 2560,
+        // 1 plane, 16 tokens 13.4 us a call, 12.0 now)
+        constexpr uint32_t kAtOnce = kCW < 32 ? kCW : 32;
 #pragma unroll 1
-        for (uint32_t c = 0; c < kCW && tok0 + c < p.m; c += 16) {
+        for (uint32_t c = 0; c < kCW && tok0 + c < p.m; c += kAtOnce) {
           const float* part = p.partial + size_t(tok0 + c) * p.n + n;
-          float sum[16];
+          float sum[kAtOnce];
 #pragma unroll
-          for (uint32_t i = 0; i < 16; ++i) sum[i] = __ldcg(part + size_t(i) * p.n);
+          for (uint32_t i = 0; i < kAtOnce; ++i) sum[i] = __ldcg(part + size_t(i) * p.n);
 #pragma unroll 1
           for (uint32_t s2 = 1; s2 < p.splits; ++s2) {
             part += size_t(p.m_pad) * p.n;
+            float more[kAtOnce];
 #pragma unroll
-            for (uint32_t i = 0; i < 16; ++i) sum[i] = __fadd_rn(sum[i], __ldcg(part + size_t(i) * p.n));
+            for (uint32_t i = 0; i < kAtOnce; ++i) more[i] = __ldcg(part + size_t(i) * p.n);
+#pragma unroll
+            for (uint32_t i = 0; i < kAtOnce; ++i) sum[i] = __fadd_rn(sum[i], more[i]);
           }
-          finish_outputs(p, sum, tok0 + c, n, rs);
+#pragma unroll
+          for (uint32_t i = 0; i < kAtOnce; i += 16) finish_outputs(p, &sum[i], tok0 + c + i, n, rs);
         }
       }
       named_sync(kBarEpilogue, 32 * kEpilogueWarps);   // the flag has been read
@@ -889,11 +902,18 @@ uint32_t tile_tokens(const tb_weights* w, uint32_t m, uint32_t sm_count) {
   const uint64_t half = waves(128), whole = waves(256);
   return half == whole || (2 * half <= 3 * whole && tile_planes <= 40) || tile_planes <= 4 ? 128 : 256;
 }
-// K splits of an output tile: as many as keep every CTA of one wave busy, at most one per tile column.
-uint32_t splits_of(const tb_weights* w, uint32_t m, uint32_t sm_count) {
-  const uint32_t tpr = uint32_t(w->k / 256), out_tiles = uint32_t((w->n + kRows - 1) / kRows);
-  if (m > 64 || out_tiles >= sm_count || out_tiles > kMaxSplitTiles) return 1;   // up to 64 tokens are one token tile
-  return std::max(1u, std::min(std::min(sm_count / out_tiles, tpr), 8u));
+// K splits of an output tile, for token tiles of up to 128: as many as keep every CTA of one wave busy, at most one
+// per tile column.  A 128-token tile passes 64 KB of sums through memory per part, about 6 us, or the time of
+// seven tile-planes: it is split where at least kWorthTilePlanes are saved.  Measured, whole / split, us: 5120 x 5120,
+// 2 planes, 100 tokens (26 saved) 44.5 / 28.3; 2560 x 2560, 3 planes, 128 tokens (24) 35.3 / 25.6; 2560 x 6912, 1 plane,
+// 200 tokens (18) 32.1 / 24.6; but 8192 x 2048, 1 plane, 128 tokens (4) 16.3 / 17.6.
+constexpr uint32_t kWorthTilePlanes = 10;
+uint32_t splits_of(const tb_weights* w, uint32_t m, uint32_t tt, uint32_t sm_count) {
+  const uint32_t tpr = uint32_t(w->k / 256), out_tiles = uint32_t((w->n + kRows - 1) / kRows) * ((m + tt - 1) / tt);
+  if (tt > 128 || out_tiles >= sm_count || out_tiles > kMaxSplitTiles) return 1;
+  const uint32_t splits = std::max(1u, std::min(std::min(sm_count / out_tiles, tpr), 8u));
+  if (tt == 128 && (tpr - (tpr + splits - 1) / splits) * w->uniform_planes < kWorthTilePlanes) return 1;
+  return splits;
 }
 
 struct Scratch { int8_t* qperm; float* ascale; float* partial; size_t fixed; };
@@ -949,11 +969,16 @@ bool tb_prefill_registers_hold(uint32_t m, int launch_regs) {
   return kernel_of(tbf::kB3, widest_tile(m), 1, false).pool_holds(launch_regs);   // the same for every codec and plane count
 }
 
+namespace {
+uint32_t sm_count_of(const tb_weights* w) { return w->owner ? uint32_t(w->owner->prop.multiProcessorCount) : 148u; }
+}  // namespace
 size_t tb_prefill_scratch_bytes(const tb_weights* w, uint32_t m) {
-  const uint32_t m_pad = pad_tokens(m);
-  const uint32_t sm_count = w->owner ? uint32_t(w->owner->prop.multiProcessorCount) : 148u;
-  const uint32_t splits = splits_of(w, m, sm_count);
-  return carve(nullptr, m_pad, uint32_t(w->k)).fixed + (splits > 1 ? size_t(splits) * m_pad * w->n * 4 : 0) + 256;
+  const uint32_t tt = tile_tokens(w, m, sm_count_of(w)), rows = (m + tt - 1) / tt * tt, splits = splits_of(w, m, tt, sm_count_of(w));
+  return carve(nullptr, pad_tokens(m), uint32_t(w->k)).fixed + (splits > 1 ? size_t(splits) * rows * w->n * 4 : 0) + 256;
+}
+// Split tiles number no more than the SMs, so the parts of all of them hold no more than an output tile per SM.
+size_t tb_prefill_reserve_bytes(const tb_weights* w, uint32_t max_m) {
+  return carve(nullptr, pad_tokens(max_m), uint32_t(w->k)).fixed + size_t(sm_count_of(w)) * std::min(widest_tile(max_m), 128u) * kRows * 4 + 256;
 }
 
 cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t stream) {
@@ -1005,9 +1030,9 @@ cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t s
   pp.payload = w->d_payload; pp.scales = w->d_scales;
   pp.ascale = sc.ascale;
   pp.y = a.y; pp.acc_dump = a.acc_dump; pp.row_scale = a.row_scale; pp.status = a.status; pp.residual = a.residual;
-  pp.m = a.m; pp.m_pad = m_pad; pp.n = uint32_t(w->n); pp.k = k; pp.tpr = k / 256; pp.y_dtype = uint32_t(a.y_dtype);
+  pp.m = a.m; pp.m_pad = rows; pp.n = uint32_t(w->n); pp.k = k; pp.tpr = k / 256; pp.y_dtype = uint32_t(a.y_dtype);
   pp.n_tiles = (pp.n + kRows - 1) / kRows; pp.m_tiles = m_tiles;
-  pp.splits = splits_of(w, a.m, uint32_t(sm_count));
+  pp.splits = splits_of(w, a.m, tt, uint32_t(sm_count));
   if (pp.splits > 1) {
     if (!a.tile_counters) return cudaErrorInvalidValue;
     pp.partial = sc.partial; pp.tile_counters = a.tile_counters;

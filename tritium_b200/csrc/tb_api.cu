@@ -580,12 +580,7 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
 
 tb_status reserve_prefill(tb_backend* b, const tb_weights* w, uint32_t m) {
   if (!w->fast || !tb_prefill_supported(w, m)) return TB_OK;
-  // batches of up to 64 tokens split K and keep partial sums in the scratch as well, so the need
-  // does not grow monotonically with m: reserve for the largest of the kernel's token-tile classes
-  size_t need = tb_prefill_scratch_bytes(w, m);
-  for (uint32_t edge : {32u, 64u})
-    if (m > edge) need = std::max(need, tb_prefill_scratch_bytes(w, edge));
-  return ensure(&b->d_q, &b->d_q_cap, need);
+  return ensure(&b->d_q, &b->d_q_cap, tb_prefill_reserve_bytes(w, m));
 }
 
 // Host-pointer wrapper: stage in, run, check, stage out.  `y` is written only on success.

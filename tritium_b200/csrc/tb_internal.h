@@ -206,6 +206,8 @@ bool tb_prefill_supported(const tb_weights* w, uint32_t m);
 // Whether the launch for `m` tokens accepts a kernel that was compiled to `launch_regs` registers per thread.
 bool tb_prefill_registers_hold(uint32_t m, int launch_regs);
 size_t tb_prefill_scratch_bytes(const tb_weights* w, uint32_t m);
+// Enough for every call of up to `max_m` tokens.
+size_t tb_prefill_reserve_bytes(const tb_weights* w, uint32_t max_m);
 cudaError_t tb_launch_prefill(const PrefillArgs& a, int sm_count, cudaStream_t stream);
 
 // peer-memory communicator (kernels_comm.cu)
