@@ -83,11 +83,11 @@ template <int TT> struct Tile {
   // CTA got at launch, threads x the registers the compiler allotted (launch bounds: 96 per thread with
   // 640 threads, 80 with 768), and a setmaxnreg.inc waits without limit for registers that the others
   // have not given back, so the shares must add up to no more than the pool:
-  //   TT = 256:  128 x 40 (copy, MMA, idle) + 256 x 160 (epilogue) + 256 x 56 (expanders) = 60,416 <= 640 x 96
+  //   TT = 256:  128 x 32 (copy, MMA, idle) + 256 x 160 (epilogue) + 256 x 64 (expanders) = 61,440  = 640 x 96
   //   else:      128 x 40 + 256 x 112 + 384 x 72                                          = 61,440  = 768 x 80
   // Another compiler or other flags may allot other counts: the launch asks the built kernel and is
   // refused unless pool_holds (a share below the launch count is given back, one above it is drawn).
-  static constexpr int kControlRegs = 40, kEpilogueRegs = TT == 256 ? 160 : 112, kExpandRegs = TT == 256 ? 56 : 72;
+  static constexpr int kControlRegs = TT == 256 ? 32 : 40, kEpilogueRegs = TT == 256 ? 160 : 112, kExpandRegs = TT == 256 ? 64 : 72;
   static constexpr bool pool_holds(int launch_regs) {
     return launch_regs >= kControlRegs && launch_regs >= kExpandRegs && launch_regs <= kEpilogueRegs &&
            32 * (kFirstEpilogueWarp * kControlRegs + kEpilogueWarps * kEpilogueRegs + kGroupWarps * kExpGroups * kExpandRegs) <= kThreads * launch_regs;
