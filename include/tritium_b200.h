@@ -192,8 +192,9 @@ tb_status tb_salt_v2_gather_rows(tb_backend* backend, const tb_weights* weights,
 #define TB_FWD_PDL 4u         /* launch with programmatic dependent launch (weights prefetch early) */
 #define TB_FWD_FORCE_DECODE 8u   /* streaming kernel whatever m; TB_UNSUPPORTED_FORMAT when a row block does not fit */
 #define TB_FWD_FORCE_PREFILL 16u /* tensor-core kernel whatever m */
-/* Without a force flag: up to 8 tokens take the streaming (decode) kernel, more the tensor-core
- * kernels; a tensor whose rows are too long for the streaming kernel's shared-memory ring takes the
+/* Without a force flag: up to 4 tokens take the streaming (decode) kernel, more the tensor-core
+ * kernels (5 to 8 tokens only in device calls where tb_backend_reserve has been called for that many, else two
+ * chained streaming passes); a tensor whose rows are too long for the streaming kernel's shared-memory ring takes the
  * tensor-core kernel at every m (so a device-pointer caller reserves with tb_backend_reserve). */
 typedef struct tb_forward_args {
   const void* x;            /* [m,k] device */

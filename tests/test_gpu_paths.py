@@ -717,3 +717,42 @@ def test_host_outputs_keep_their_memory(m):
     for got, i in zip(kept, (0, 2, 3)):
         assert rel_l2(got, want[i]) <= 1e-5 and got.flags.writeable and got.shape == (m, n)
     assert np.array_equal(exact.view(np.uint32), want[0].view(np.uint32))
+
+
+@pytest.mark.parametrize("k", [768, 2560])
+@pytest.mark.parametrize("m", [5, 8])
+def test_five_to_eight_tokens_with_and_without_reserved_scratch(k, m):
+    """Device calls of five to eight tokens take the tensor cores where scratch for them is reserved and two decode
+    passes where it is not (nothing is allocated then: the call can be captured).  Both against the oracle, with a
+    norm and a residual too."""
+    import torch
+    from tritium_b200 import B200Backend
+    n = 300
+    prod, orac = uniform_pair(n, k, 2, seed=k)
+    x = make_activations(m, k, seed=m, bf16=True)
+    want, want_acc, _ = orc.a8_linear(orac, x, dump=True)
+    weight = (1 + 0.1 * np.random.default_rng(3).standard_normal(k)).astype(np.float32)
+    residual = torch.randn(m, n, device="cuda")
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(weight).cuda()
+    normed = orc.a8_linear(orac, orc.rmsnorm(x, weight, 1e-6), dump=False)[0]
+    for reserved in (False, True):
+        b = B200Backend(0)
+        resident = b.upload_salt_v2(prod, SaltV2Codec.B3)
+        if reserved:
+            b.reserve(resident, m)
+        y, dump = torch.zeros(m, n, device="cuda"), torch.zeros(m, n, k // 128, 2, dtype=torch.int32, device="cuda")
+        y2, y3 = torch.zeros_like(y), torch.zeros_like(y)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            b.forward_dev(resident, xd, y, acc_dump=dump)
+        graph.replay()
+        b.norm_linear_forward_dev(resident, xd, y2, norm_weight=wd, eps=1e-6)
+        b.norm_linear_forward_dev(resident, xd, y3, norm_weight=wd, eps=1e-6, residual=residual)
+        b.check()
+        assert np.array_equal(dump.cpu().numpy(), want_acc[..., :2])
+        assert rel_l2(y.cpu().numpy(), want) <= 1e-5 and rel_l2(y2.cpu().numpy(), normed) <= 1e-5
+        assert torch.equal(y3, residual + y2)
+        del graph
+        resident.free()
+        b.close()

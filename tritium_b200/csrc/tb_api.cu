@@ -417,6 +417,15 @@ tb_status reserve_prefill(tb_backend* b, const tb_weights* w, uint32_t m);
 bool decode_fits(const tb_backend* b, const tb_weights* w, uint32_t m) {
   return tb_decode_supported(w, std::min<uint32_t>(std::max<uint32_t>(m, 1u), 4u), b->max_smem_optin, nullptr);
 }
+// Five to eight tokens: two chained decode passes or one tensor-core call.  Measured, us per call in a graph, decode /
+// tensor cores at 5 and 8 tokens (B3): 1024 x 1024, 1 plane 10.4 / 9.5, 11.0 / 9.2; 2560 x 2560, 1 plane 14.3 / 11.9,
+// 15.3 / 11.5; 6912 x 2560, 3 planes 22.1 / 17.6, 22.8 / 17.6; 34816 x 5120, 2 planes 66 / 51, 72 / 51; D2 alike.  The
+// decode passes win only where three B3 planes meet a last wave of row tiles that is nearly empty: 20000 x 4096,
+// 3 planes (157 tiles on 148 SMs) 50 / 63.
+bool two_passes_win(const tb_backend* b, const tb_weights* w) {
+  const uint64_t sms = uint64_t(b->prop.multiProcessorCount), tiles = (w->n + 127) / 128, slots = (tiles + sms - 1) / sms * sms;
+  return w->uniform_planes == 3 && w->codec == tbf::kB3 && tiles > sms && tiles * 100 < slots * 55;
+}
 bool takes_tensor_cores(const tb_backend* b, const tb_weights* w, uint32_t m, uint32_t flags, uint32_t decode_limit = 8) {
   if (flags & TB_FWD_FORCE_PREFILL) return true;
   if (flags & TB_FWD_FORCE_DECODE) return false;
@@ -432,7 +441,7 @@ struct BlockExtras {
 
 // Device-pointer dispatch shared by every entry point.  Returns the kernel family used.
 tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args& a_in, cudaStream_t st, tb_receipt* receipt,
-                      const BlockExtras& ex = BlockExtras{}) {
+                      const BlockExtras& ex = BlockExtras{}, bool device_call = false) {
   tb_forward_args a = a_in;
   if (a.m == 0 || w->n == 0) { fill_receipt(w, 0, 0, 0, 0, 0, receipt); return TB_OK; }
   if (!a.x || !a.y) return tb_fail(TB_NULL_ARG, "null activation or output pointer");
@@ -502,12 +511,16 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
     fill_receipt(w, a.m, dtype_size(a.x_dtype), dtype_size(a.y_dtype), 0, ex.norm_weight ? 4 : 3, receipt);
     return TB_OK;
   }
-  // One or two chained decode passes (up to 4 or 8 tokens), else the tensor cores.  Measured with flushed
-  // caches, us, decode / tensor cores, at 4, 5 and 8 tokens: 6912 x 2560, 3 planes 23.5 / 23.5, 37.9 / 23.5,
-  // 33.8 / 23.5; 2560 x 2560, 1 plane 15.6 / 19.4, 27.6 / 19.4, 25.6 / 17.4; 34816 x 5120, 2 planes 48 / 60,
-  // 87 / 60, 87 / 60.  So one pass is level or faster; the limit of two passes was drawn when the
-  // tensor-core kernel took 25 us where it takes 20 now, and two passes lose by a third today.
-  const bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags);
+  // Up to four tokens one decode pass, from nine on the tensor cores.  Measured with flushed caches, us, decode /
+  // tensor cores at 4 tokens: 6912 x 2560, 3 planes 23.5 / 23.5; 2560 x 2560, 1 plane 15.6 / 19.4; 34816 x 5120, 2 planes
+  // 48 / 60.  In between the tensor cores too (see two_passes_win), if what they need is reserved: a caller that has
+  // reserved nothing keeps the two decode passes, and so do the host calls, whose copies outweigh the difference, and rows
+  // of up to 1,024 columns where a norm or programmatic dependent launch goes with them.
+  bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags);
+  if (device_call && !want_prefill && a.m > 4 && !(a.flags & TB_FWD_FORCE_DECODE) && !two_passes_win(b, w))
+    want_prefill = tb_prefill_supported(w, a.m) && b->d_q_cap >= tb_prefill_scratch_bytes(w, a.m) &&
+                   (!ex.norm_weight || b->d_norm_cap >= size_t(a.m) * w->k * 4) &&
+                   !((ex.norm_weight || (a.flags & TB_FWD_PDL)) && w->k <= 1024);
   uint32_t extra_launches = 0;
   // The decode kernel normalises inside its table builder.  Every other route (the tensor-core
   // kernel, tables from the preparation kernel) takes rows normalised by a kernel of its own; the
@@ -580,6 +593,8 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
 
 tb_status reserve_prefill(tb_backend* b, const tb_weights* w, uint32_t m) {
   if (!w->fast || !tb_prefill_supported(w, m)) return TB_OK;
+  // normalised rows of calls of a few tokens (see forward_dev)
+  if (m > 4) if (tb_status s = ensure(&b->d_norm, &b->d_norm_cap, size_t(std::min(m, 8u)) * w->k * 4)) return s;
   return ensure(&b->d_q, &b->d_q_cap, tb_prefill_reserve_bytes(w, m));
 }
 
@@ -678,7 +693,7 @@ extern "C" tb_status tb_linear_forward_dev(tb_backend* b, const tb_weights* w, c
   if (!args) return tb_fail(TB_NULL_ARG, "args is null");
   if (tb_status s = use_device(b)) return s;
   cudaStream_t st = args->stream ? static_cast<cudaStream_t>(args->stream) : b->stream;
-  return forward_dev(b, w, *args, st, receipt);
+  return forward_dev(b, w, *args, st, receipt, BlockExtras{}, true);
 }
 
 extern "C" tb_status tb_norm_linear_forward_dev(tb_backend* b, const tb_weights* w, const tb_norm_linear_args* args, tb_receipt* receipt) {
@@ -698,7 +713,7 @@ extern "C" tb_status tb_norm_linear_forward_dev(tb_backend* b, const tb_weights*
   ex.norm_weight = args->norm_weight; ex.norm_eps = args->norm_eps;
   ex.norm_zero_centered = (args->norm_flags & TB_NORM_ZERO_CENTERED) != 0; ex.residual = args->residual;
   ex.relu2_up = args->relu2_up;
-  return forward_dev(b, w, a, st, receipt, ex);
+  return forward_dev(b, w, a, st, receipt, ex, true);
 }
 
 extern "C" tb_status tb_act_absmax_dev(tb_backend* b, const void* x, tb_dtype x_dtype, uint32_t m, uint32_t k, float* out, void* stream) {
