@@ -1294,8 +1294,11 @@ bool tb_decode_builds_tables(const tb_weights* w, uint32_t m, const void* x) {
   // (5120 x 5120), 27 pairs 9.2 / 9.7 (2560 x 6912), 68 pairs 26.5 / 21.8 (5120 x 17408); four tokens, 40 pairs
   // 15.2 / 12.1, 80 pairs 18.1 / 12.1.  Level at 20 pairs, where the second launch costs the host 2 us besides; a
   // four-token table has twice the entries per pair and goes by one pass of the builder.
+  // D2 leaves the launch less time for the builder to hide in: 25 pairs 19.0 / 18.5 (30848 x 6400, one token), layers of
+  // 1,024 columns at 8 tokens (16 pairs) 160 / 152 us, where B3 takes 166 / 176.
   const uint32_t mk = layout_tokens(m), pairs = uint32_t(w->k / 256) * mk;
-  return pairs <= (use_dual(mk) ? 32u : 16u) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  const uint32_t most = w->codec == tbf::kD2 ? 12u : use_dual(mk) ? 32u : 16u;
+  return pairs <= most && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
 }
 
 cudaError_t tb_launch_prepare(const DecodeArgs& a, cudaStream_t stream) {
