@@ -719,6 +719,7 @@ __device__ __forceinline__ void epilogue_role(const PrefillParams& p, uint32_t t
       if (tp + 1 < tp_end) fetch_scale(tp + 1);
       if (!live) {   // nothing but padding tokens in this half: hand the accumulator back
         mbar_wait(full0 + 8 * buf, parity, wctx, 306);
+        __syncwarp();   // a lane that still polls would miss this phase once the accumulator is refilled
         if (lane == 0) mbar_arrive(empty0 + 8 * buf);
       } else
 #pragma unroll
