@@ -56,8 +56,8 @@ struct DecodeParams {
   const uint8_t* payload; const uint16_t* scales;   // single layer (layers == nullptr)
   const TbLayerDesc* layers; uint32_t layer_count; uint32_t y_layer_stride;   // grouped launch: outputs [layer][m][n]
   const uint8_t* tables; uint32_t table_bytes;   // z tables | accumulator start values | token scales
-  // fused prologue (fused != 0): the CTA quantises x and builds its tables itself
-  const void* x; const float* act_scale_in; const float* act_absmax_in; uint32_t x_dtype, fused;
+  // fused prologue (kernels with BUILD): the CTA quantises x and builds its tables itself
+  const void* x; const float* act_scale_in; const float* act_absmax_in; uint32_t x_dtype;
   // fused RMSNorm in front of the quantiser (fused launches only; null = none) and `residual + y`
   // behind the token scale (fp32, indexed like y; null = none)
   const float* norm_weight; float norm_eps; uint32_t norm_zero_centered;
@@ -769,7 +769,13 @@ __device__ __forceinline__ void build_tables(const DecodeParams& p, uint8_t* sme
 // ---------------------------------------------------------------- the kernel
 // M: token columns the tables are laid out for (1, 2 or 4; p.m <= M tokens are valid).
 // SETS: blocks of 16 row-planes in one row block (rows_per_stage * PLANES / 16).
-template <int CODEC, int PLANES, int M, int SETS>
+// BUILD: the kernel builds its activation tables itself (else it reads those of prepare_kernel).  Two kernels,
+// because the builder takes 90 to 96 registers per thread where the main loop of small row blocks takes 70 to 77:
+// without it the CTAs of two launches leave the registers that a preparation kernel needs to start beside
+// them, and a chain of dependent launches overlaps.  One kernel for both / two, us a call of such a chain: 2688 x 2048,
+// 2 planes, 3 tokens, B3 7.3 / 6.1; 11264 x 2048, 2 planes, 4 tokens, D2 9.6 / 8.4; four decoder layers of 2,048 columns,
+// 2 planes, 4 tokens, B3 172 / 158.
+template <int CODEC, int PLANES, int M, int SETS, bool BUILD>
 __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams p) {
   using T = Traits<CODEC>;
   constexpr bool DUAL = M <= 2;
@@ -810,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   // builds its own tables shares no scratch with its neighbours, so it raises the trigger at
   // once.  A launch that waits for tables in global scratch raises it only after that wait, so
   // that a later launch which shares the tables (and does not wait) cannot outrun them.
-  if (p.pdl && (p.fused || !p.wait_tables)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.pdl && (BUILD || !p.wait_tables)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   const uint32_t total_blocks = p.blocks * p.layer_count;
   const uint32_t my_blocks = blockIdx.x < total_blocks ? (total_blocks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -966,7 +972,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   }
 
   // -------------------------------------------------- consumers: activation tables
-  if (p.fused) {
+  if constexpr (BUILD) {
     clear_tables(p, smem, tid);
     consumer_sync();
     // x may be the previous kernel's output: wait for it (the weight stream is already running)
@@ -1332,14 +1338,24 @@ cudaError_t tb_launch_prepare(const DecodeArgs& a, cudaStream_t stream) {
 }
 
 using DecodeKernel = void (*)(const DecodeParams);
-template <int CODEC, int PLANES, int SETS> DecodeKernel pick_tokens(uint32_t mk) {
-  return mk == 1 ? decode_kernel<CODEC, PLANES, 1, SETS> : mk == 2 ? decode_kernel<CODEC, PLANES, 2, SETS> : decode_kernel<CODEC, PLANES, 4, SETS>;
+template <int CODEC, int PLANES, int SETS, bool BUILD> DecodeKernel pick_tokens(uint32_t mk) {
+  return mk == 1   ? decode_kernel<CODEC, PLANES, 1, SETS, BUILD>
+         : mk == 2 ? decode_kernel<CODEC, PLANES, 2, SETS, BUILD>
+                   : decode_kernel<CODEC, PLANES, 4, SETS, BUILD>;
 }
-template <int CODEC, int PLANES> DecodeKernel pick_sets(uint32_t sets, uint32_t mk) {
-  return sets == 1 ? pick_tokens<CODEC, PLANES, 1>(mk) : sets == 2 ? pick_tokens<CODEC, PLANES, 2>(mk) : pick_tokens<CODEC, PLANES, 4>(mk);
+template <int CODEC, int PLANES, bool BUILD> DecodeKernel pick_sets(uint32_t sets, uint32_t mk) {
+  return sets == 1   ? pick_tokens<CODEC, PLANES, 1, BUILD>(mk)
+         : sets == 2 ? pick_tokens<CODEC, PLANES, 2, BUILD>(mk)
+                     : pick_tokens<CODEC, PLANES, 4, BUILD>(mk);
 }
-template <int CODEC> DecodeKernel pick_planes(uint32_t planes, uint32_t sets, uint32_t mk) {
-  return planes == 1 ? pick_sets<CODEC, 1>(sets, mk) : planes == 2 ? pick_sets<CODEC, 2>(sets, mk) : pick_tokens<CODEC, 3, 3>(mk);
+template <int CODEC, bool BUILD> DecodeKernel pick_planes(uint32_t planes, uint32_t sets, uint32_t mk) {
+  return planes == 1   ? pick_sets<CODEC, 1, BUILD>(sets, mk)
+         : planes == 2 ? pick_sets<CODEC, 2, BUILD>(sets, mk)
+                       : pick_tokens<CODEC, 3, 3, BUILD>(mk);
+}
+DecodeKernel pick_kernel(int codec, uint32_t planes, uint32_t sets, uint32_t mk, bool build) {
+  if (codec == tbf::kB3) return build ? pick_planes<tbf::kB3, true>(planes, sets, mk) : pick_planes<tbf::kB3, false>(planes, sets, mk);
+  return build ? pick_planes<tbf::kD2, true>(planes, sets, mk) : pick_planes<tbf::kD2, false>(planes, sets, mk);
 }
 
 cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cudaStream_t stream) {
@@ -1355,7 +1371,7 @@ cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cu
     if (a.comm_absmax && !a.comm_y) return cudaErrorInvalidValue;
     if (a.comm_y && a.comm_y->world > 1 && !a.comm_absmax && !a.act_absmax_in && a.x_dtype != TB_I8) return cudaErrorInvalidValue;
     if (a.x_dtype == TB_I8 && !a.act_scale_in) return cudaErrorInvalidValue;
-    p.fused = 1; p.x = a.x; p.act_scale_in = a.act_scale_in; p.act_absmax_in = a.act_absmax_in; p.x_dtype = uint32_t(a.x_dtype);
+    p.x = a.x; p.act_scale_in = a.act_scale_in; p.act_absmax_in = a.act_absmax_in; p.x_dtype = uint32_t(a.x_dtype);
     if (a.relu2_up) {
       if (a.x_dtype != TB_F32 || (reinterpret_cast<uintptr_t>(a.relu2_up) & 15u) || a.norm_weight) return cudaErrorInvalidValue;
       p.relu2_up = a.relu2_up;
@@ -1394,7 +1410,7 @@ cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cu
   p.wait_tables = a.tables_shared ? 0u : 1u;
   p.inject_missing_tx = a.inject_missing_tx;
   const uint32_t sets = w->plan.rows_per_stage * w->uniform_planes / 16, mk = layout_tokens(a.m);
-  DecodeKernel kernel = w->codec == tbf::kB3 ? pick_planes<tbf::kB3>(w->uniform_planes, sets, mk) : pick_planes<tbf::kD2>(w->uniform_planes, sets, mk);
+  DecodeKernel kernel = pick_kernel(w->codec, w->uniform_planes, sets, mk, a.fused);
   if (!kernel) return cudaErrorInvalidConfiguration;
   if (a.layers && a.layer_count > uint32_t(kMaxGroupLayers)) return cudaErrorInvalidValue;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
