@@ -274,7 +274,9 @@ tb_status tb_linear_forward_a8_static(tb_backend* backend, const tb_weights* wei
 tb_status tb_act_absmax_dev(tb_backend* backend, const void* x, tb_dtype x_dtype, uint32_t m, uint32_t k,
                             float* out, void* stream);
 /* Reserves the backend's device scratch for `weights` at up to `max_m` tokens, so that later
- * tb_linear_forward_dev calls allocate nothing. */
+ * tb_linear_forward_dev calls allocate nothing.  Scratch may be replaced by a larger buffer in any later call, but a
+ * buffer that a captured launch uses is kept until the backend is freed: a CUDA graph stays valid whatever is
+ * reserved or called after it was recorded. */
 tb_status tb_backend_reserve(tb_backend* backend, const tb_weights* weights, uint32_t max_m);
 /* Reads and clears the device status word written by bounded waits / finite checks. */
 tb_status tb_backend_check(tb_backend* backend, void* stream);

@@ -9,7 +9,7 @@ import pytest
 
 from oracle import oracle as orc
 from tritium_b200 import _lib, errors
-from tritium_b200.format import SaltV2Codec
+from tritium_b200.format import SaltV2Codec, SaltV2Tensor
 from tritium_b200.synth import bf16_bits_to_f32, f32_to_bf16_bits, make_activations
 
 from gpu_common import exact_group_sums, rel_l2, uniform_pair
@@ -756,3 +756,64 @@ def test_five_to_eight_tokens_with_and_without_reserved_scratch(k, m):
         del graph
         resident.free()
         b.close()
+
+
+def test_graphs_outlive_later_reservations_and_calls():
+    """Captured calls on the backend's scratch (five and eight tokens, norm in front of prepared tables, fp32 activations, a
+    layout without a fast kernel) give the same bits after larger reservations and host calls, with whatever those
+    freed filled with ones."""
+    import torch
+    from tritium_b200 import B200Backend
+    b = B200Backend(0)
+    small, _ = uniform_pair(300, 2560, 2, seed=1)
+    large, _ = uniform_pair(1500, 8448, 1, seed=2)
+    rng = np.random.default_rng(3)
+    scales = np.full((60, 3, 4), np.float16(0.05).view(np.uint16))
+    ragged = SaltV2Tensor("w", 40, 384, np.full(60, 3, np.uint8), rng.integers(-1, 2, (60, 3, 256)).astype(np.int8), scales, 64)
+    w, wl, wr = (b.upload_salt_v2(t, SaltV2Codec.B3) for t in (small, large, ragged))
+    b.reserve(w, 8)
+    weight = {k: torch.rand(k, device="cuda") + 0.5 for k in (2560, 8448)}
+    calls = []
+    for wt, n, k, m in ((w, 300, 2560, 5), (w, 300, 2560, 8), (wl, 1500, 8448, 1), (w, 300, 2560, 2), (wr, 40, 384, 3)):
+        calls.append((wt, torch.randn(m, k, device="cuda"), torch.zeros(m, n, device="cuda"), k))
+
+    def run(i):
+        wt, x, y, k = calls[i]
+        if i in (1, 2):
+            b.norm_linear_forward_dev(wt, x, y, norm_weight=weight[k], eps=1e-6)
+        else:
+            b.forward_dev(wt, x, y, a8=i != 3)
+
+    graphs, first = [], []
+    for i in range(len(calls)):
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            run(i)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run(i)
+        graph.replay()
+        torch.cuda.synchronize()
+        graphs.append(graph)
+        first.append(calls[i][2].clone())
+        assert first[-1].abs().sum() > 0
+    b.check()
+    b.reserve(wl, 2048)
+    b.linear_forward_a8(wl, np.ones((8, 8448), np.float32), 8)
+    b.salt_v2_forward_fast(wl, np.ones((64, 8448), np.float32), 64)
+    b.linear_forward_a8(wr, np.ones((200, 384), np.float32), 200)
+    torch.cuda.synchronize()
+    filler = [torch.ones(1 << 20, device="cuda") for _ in range(64)]
+    for (_, _, y, _), graph, want in zip(calls, graphs, first):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+    b.check()
+    assert all(bool((f == 1).all()) for f in filler)
+    graphs.clear()
+    for h in (w, wl, wr):
+        h.free()
+    b.close()

@@ -66,6 +66,32 @@ tb_status ensure(void** ptr, size_t* cap, size_t need, bool pinned_host = false)
   return TB_OK;
 }
 
+// The same for scratch of device calls, whose address a CUDA graph may hold (tb_scratch.h).
+tb_status ensure(tb_backend* b, tb_scratch* s, size_t need) {
+  cudaError_t err = cudaSuccess;
+  const auto alloc = [&](size_t bytes) {
+    void* p = nullptr;
+    err = cudaMalloc(&p, bytes);
+    return err == cudaSuccess ? p : nullptr;
+  };
+  if (tb_scratch_grow(s, &b->kept, need, alloc, [](void* p) { cudaFree(p); })) return TB_OK;
+  return tb_cuda_fail(err == cudaSuccess ? cudaErrorMemoryAllocation : err, "allocate scratch");
+}
+// `s` is used by a launch on `st`: remember it when that launch goes into a graph.  Where the question fails
+// (the legacy stream beside a capture: the launch will fail too) the answer is taken to be yes.
+void* on_stream(tb_scratch* s, cudaStream_t st) {
+  if (!s->recorded) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+      cudaGetLastError();
+      s->recorded = true;
+    } else if (status != cudaStreamCaptureStatusNone) {
+      s->recorded = true;
+    }
+  }
+  return s->ptr;
+}
+
 tb_status use_device(const tb_backend* b) {
   TB_CUDA(cudaSetDevice(b->ordinal), "select device");
   return TB_OK;
@@ -181,7 +207,9 @@ void destroy_backend(tb_backend* b) {
   cudaSetDevice(b->ordinal);
   if (b->stream) { cudaStreamSynchronize(b->stream); cudaStreamDestroy(b->stream); }
   cudaFree(b->d_status); cudaFreeHost(b->h_status);
-  cudaFree(b->d_x); cudaFree(b->d_y); cudaFree(b->d_aux); cudaFree(b->d_q); cudaFree(b->d_prep); cudaFree(b->d_norm); cudaFree(b->d_limb); cudaFree(b->d_tile_counters); cudaFreeHost(b->h_pin);
+  cudaFree(b->d_x); cudaFree(b->d_y); cudaFree(b->d_aux); cudaFree(b->q.ptr); cudaFree(b->d_prep); cudaFree(b->norm.ptr); cudaFree(b->limb.ptr); cudaFree(b->d_tile_counters);
+  for (void* p : b->kept) cudaFree(p);
+  cudaFreeHost(b->h_pin);
   delete b;
 }
 }  // namespace
@@ -461,9 +489,9 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
       // kernels (exact int32 sums per limb), the four outputs of a token added in a fixed order.
       const uint32_t m4 = a.m * 4;
       const size_t qb = (size_t(m4) * w->k + 255) & ~size_t(255), sb = (size_t(m4) * 4 + 255) & ~size_t(255);
-      if (tb_status s = ensure(&b->d_limb, &b->d_limb_cap, qb + sb + size_t(m4) * w->n * 4 + 256)) return s;
+      if (tb_status s = ensure(b, &b->limb, qb + sb + size_t(m4) * w->n * 4 + 256)) return s;
       if (takes_tensor_cores(b, w, m4, a.flags)) if (tb_status s = reserve_prefill(b, w, m4)) return s;
-      uint8_t* base = static_cast<uint8_t*>(b->d_limb);
+      uint8_t* base = static_cast<uint8_t*>(on_stream(&b->limb, st));
       int8_t* q = reinterpret_cast<int8_t*>(base);
       float* scales = reinterpret_cast<float*>(base + qb);
       float* y4 = reinterpret_cast<float*>(base + qb + sb);
@@ -493,8 +521,8 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
     if (a.acc_dump) return tb_fail(TB_UNSUPPORTED_FORMAT, "the accumulator dump needs uniform plane counts, k % 256 == 0, group 128 and codec D2 or B3");
     if (a.x_dtype == TB_I8 || a.act_absmax) return tb_fail(TB_UNSUPPORTED_FORMAT, "this layout takes fp32 or bf16 activations without a supplied absmax");
     const size_t qf = (size_t(a.m) * w->k * 4 + 255) & ~size_t(255), yf = (size_t(a.m) * w->n * 4 + 255) & ~size_t(255);
-    if (tb_status s = ensure(&b->d_norm, &b->d_norm_cap, 2 * qf + yf + size_t(a.m) * 4 + 256)) return s;
-    uint8_t* base = static_cast<uint8_t*>(b->d_norm);
+    if (tb_status s = ensure(b, &b->norm, 2 * qf + yf + size_t(a.m) * 4 + 256)) return s;
+    uint8_t* base = static_cast<uint8_t*>(on_stream(&b->norm, st));
     float* q = reinterpret_cast<float*>(base + qf);           // the first qf bytes may hold normalised rows
     float* y32 = reinterpret_cast<float*>(base + 2 * qf);
     float* scale = reinterpret_cast<float*>(base + 2 * qf + yf);
@@ -518,16 +546,16 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
   // of up to 1,024 columns where a norm or programmatic dependent launch goes with them.
   bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags);
   if (device_call && !want_prefill && a.m > 4 && !(a.flags & TB_FWD_FORCE_DECODE) && !two_passes_win(b, w))
-    want_prefill = tb_prefill_supported(w, a.m) && b->d_q_cap >= tb_prefill_scratch_bytes(w, a.m) &&
-                   (!ex.norm_weight || b->d_norm_cap >= size_t(a.m) * w->k * 4) &&
+    want_prefill = tb_prefill_supported(w, a.m) && b->q.cap >= tb_prefill_scratch_bytes(w, a.m) &&
+                   (!ex.norm_weight || b->norm.cap >= size_t(a.m) * w->k * 4) &&
                    !((ex.norm_weight || (a.flags & TB_FWD_PDL)) && w->k <= 1024);
   uint32_t extra_launches = 0;
   // The decode kernel normalises inside its table builder.  Every other route (the tensor-core
   // kernel, tables from the preparation kernel) takes rows normalised by a kernel of its own; the
   // arithmetic is the same, so the codes are too.
   const auto normalise = [&](uint32_t m0, uint32_t mc) -> tb_status {
-    if (tb_status s = ensure(&b->d_norm, &b->d_norm_cap, size_t(a.m) * w->k * 4)) return s;
-    float* dst = static_cast<float*>(b->d_norm) + size_t(m0) * w->k;
+    if (tb_status s = ensure(b, &b->norm, size_t(a.m) * w->k * 4)) return s;
+    float* dst = static_cast<float*>(on_stream(&b->norm, st)) + size_t(m0) * w->k;
     const uint8_t* src = static_cast<const uint8_t*>(a_in.x) + size_t(m0) * w->k * dtype_size(a_in.x_dtype);
     TB_CUDA(tb_launch_rmsnorm(src, a_in.x_dtype, ex.norm_weight, ex.norm_eps, ex.norm_zero_centered, mc, uint32_t(w->k), dst, st),
             "launch rmsnorm");
@@ -536,13 +564,13 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
   };
   if (want_prefill && tb_prefill_supported(w, a.m)) {
     const size_t need = tb_prefill_scratch_bytes(w, a.m);
-    if (b->d_q_cap < need) return tb_fail(TB_OUT_OF_MEMORY, "prefill scratch is not reserved; call through a host entry point or tb_stack first");
+    if (b->q.cap < need) return tb_fail(TB_OUT_OF_MEMORY, "prefill scratch is not reserved; call through a host entry point or tb_stack first");
     if (ex.norm_weight) {
       if (tb_status s = normalise(0, a.m)) return s;
-      a.x = b->d_norm; a.x_dtype = TB_F32;
+      a.x = b->norm.ptr; a.x_dtype = TB_F32;
     }
     PrefillArgs pa{w, a.x, a.x_dtype, a.act_scale, a.act_absmax, a.m, a.y, a.y_dtype, a.acc_dump, a.row_scale,
-                   b->d_q, b->d_q_cap, b->d_status};
+                   on_stream(&b->q, st), b->q.cap, b->d_status};
     pa.residual = ex.residual; pa.tile_counters = b->d_tile_counters; pa.relu2_up = ex.relu2_up;
     TB_CUDA(tb_launch_prefill(pa, b->prop.multiProcessorCount, st), "launch prefill");
     fill_receipt(w, a.m, dtype_size(a_in.x_dtype), dtype_size(a.y_dtype), 2, 2 + extra_launches, receipt);
@@ -568,7 +596,7 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
         d.norm_weight = ex.norm_weight; d.norm_eps = ex.norm_eps; d.norm_zero_centered = ex.norm_zero_centered;
       } else {
         if (tb_status s = normalise(m0, mc)) return s;
-        d.x = static_cast<const float*>(b->d_norm) + size_t(m0) * w->k; d.x_dtype = TB_F32;
+        d.x = static_cast<const float*>(b->norm.ptr) + size_t(m0) * w->k; d.x_dtype = TB_F32;
       }
     }
     d.residual = ex.residual ? ex.residual + size_t(m0) * w->n : nullptr;
@@ -593,9 +621,7 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
 
 tb_status reserve_prefill(tb_backend* b, const tb_weights* w, uint32_t m) {
   if (!w->fast || !tb_prefill_supported(w, m)) return TB_OK;
-  // normalised rows of calls of a few tokens (see forward_dev)
-  if (m > 4) if (tb_status s = ensure(&b->d_norm, &b->d_norm_cap, size_t(std::min(m, 8u)) * w->k * 4)) return s;
-  return ensure(&b->d_q, &b->d_q_cap, tb_prefill_reserve_bytes(w, m));
+  return ensure(b, &b->q, tb_prefill_reserve_bytes(w, m));
 }
 
 // Host-pointer wrapper: stage in, run, check, stage out.  `y` is written only on success.
@@ -809,7 +835,10 @@ extern "C" tb_status tb_backend_reserve(tb_backend* b, const tb_weights* w, uint
   clear_error();
   if (tb_status s = check_handles(b, w)) return s;
   if (tb_status s = use_device(b)) return s;
-  return reserve_prefill(b, w, max_m);
+  if (tb_status s = reserve_prefill(b, w, max_m)) return s;
+  // normalised rows of calls of five to eight tokens (see forward_dev)
+  if (max_m > 4 && w->fast && tb_prefill_supported(w, max_m)) return ensure(b, &b->norm, size_t(std::min(max_m, 8u)) * w->k * 4);
+  return TB_OK;
 }
 
 extern "C" tb_status tb_gemm_registers_check(uint32_t m, uint32_t registers) {

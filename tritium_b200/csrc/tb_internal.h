@@ -7,9 +7,11 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "../../include/tritium_b200.h"
 #include "tb_format.h"
+#include "tb_scratch.h"
 
 // Device status word layout (uint32 x 8), written by kernels, read by tb_backend_check.
 enum : uint32_t {
@@ -38,13 +40,14 @@ struct tb_backend {
   void* d_aux = nullptr; size_t d_aux_cap = 0;   // act scales / row scales / acc dump
   void* h_pin = nullptr; size_t h_pin_cap = 0;   // pinned bounce buffer
   // scratch for the prefill path: quantised activations (permuted int8) + token scales
-  void* d_q = nullptr; size_t d_q_cap = 0;
+  tb_scratch q;
   // scratch for the decode path: activation tables built by the prepare kernel
   void* d_prep = nullptr; size_t d_prep_cap = 0;
   // normalised activations, for norm+linear calls whose tables the decode kernel does not build itself
-  void* d_norm = nullptr; size_t d_norm_cap = 0;
+  tb_scratch norm;
   // fp32 activations split into int8 limbs, their multipliers and the limbs' outputs
-  void* d_limb = nullptr; size_t d_limb_cap = 0;
+  tb_scratch limb;
+  std::vector<void*> kept;   // outgrown scratch that a CUDA graph may still use, freed with the backend
   uint32_t* d_tile_counters = nullptr;   // 256 words, zero between launches (the tensor-core kernel's K splits)
   int max_smem_optin = 0;
   // Weights, stacks and communicators point back at their backend.  tb_backend_free only marks
