@@ -817,3 +817,54 @@ def test_graphs_outlive_later_reservations_and_calls():
     for h in (w, wl, wr):
         h.free()
     b.close()
+
+
+def device_receipt(backend, resident, x, y, flags=0):
+    """Receipt of one device call: kernel 1 decode, 2 tensor cores."""
+    import ctypes as C
+    import torch
+    args = _lib.ForwardArgs()
+    args.x, args.x_dtype, args.m = x.data_ptr(), _lib.TB_F32, x.shape[0]
+    args.y, args.y_dtype, args.flags = y.data_ptr(), _lib.TB_F32, _lib.TB_FWD_A8 | flags
+    args.stream = _lib.stream_handle(torch.cuda.current_stream())
+    r = _lib.Receipt()
+    assert backend._L.tb_linear_forward_dev(backend._h, resident._h, C.byref(args), C.byref(r)) == 0
+    return r
+
+
+@pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
+@pytest.mark.parametrize("n,k,planes,tensor_cores", [(4096, 768, 1, False), (2048, 1024, 2, False), (2049, 1024, 2, True), (300, 1280, 2, True),
+                                                     (18944, 1792, 3, True), (18945, 1792, 3, None)])
+def test_kernel_of_five_to_eight_tokens_follows_the_tensors_own_reservation(codec, n, k, planes, tensor_cores):
+    """The kernel of a call of five to eight tokens depends on the tensor and on what was reserved for it: not on other
+    tensors' reservations, host calls or launch flags.  None: only B3 keeps the decode passes (a second wave of row
+    tiles that is nearly empty).  An unrelated reservation changes no bit."""
+    import torch
+    from gpu_common import product_only
+    from tritium_b200 import B200Backend
+    b = B200Backend(0)
+    w = b.upload_salt_v2(product_only(n, k, planes, seed=1), codec)
+    other = b.upload_salt_v2(product_only(512, 8192, 2, seed=2), codec)
+    if tensor_cores is None:
+        tensor_cores = codec != SaltV2Codec.B3
+    x, y = torch.randn(8, k, device="cuda"), torch.zeros(8, n, device="cuda")
+    assert device_receipt(b, w, x, y).kernel == 1
+    before = y.clone()
+    assert device_receipt(b, w, x[:6], y[:6]).kernel == 1
+    before_six = y[:6].clone()                              # passes of four and two tokens, where eight take four and four
+    b.reserve(other, 2048)
+    b.linear_forward_a8(w, np.ones((64, k), np.float32), 64)
+    assert device_receipt(b, w, x, y).kernel == 1 and torch.equal(y, before)
+    b.reserve(w, 6)
+    assert device_receipt(b, w, x, y).kernel == 1 and torch.equal(y, before)          # eight tokens are not reserved
+    for m in (5, 6):
+        for flags in (0, _lib.TB_FWD_PDL):
+            assert device_receipt(b, w, x[:m], y[:m], flags).kernel == (2 if tensor_cores else 1)
+    assert device_receipt(b, w, x[:6], y[:6], _lib.TB_FWD_FORCE_DECODE).kernel == 1
+    assert torch.equal(y[:6], before_six)
+    assert device_receipt(b, w, x[:4], y[:4]).kernel == 1
+    assert device_receipt(b, w, torch.zeros(9, k, device="cuda"), torch.zeros(9, n, device="cuda")).kernel == 2
+    b.check()
+    for h in (w, other):
+        h.free()
+    b.close()

@@ -445,14 +445,21 @@ tb_status reserve_prefill(tb_backend* b, const tb_weights* w, uint32_t m);
 bool decode_fits(const tb_backend* b, const tb_weights* w, uint32_t m) {
   return tb_decode_supported(w, std::min<uint32_t>(std::max<uint32_t>(m, 1u), 4u), b->max_smem_optin, nullptr);
 }
-// Five to eight tokens: two chained decode passes or one tensor-core call.  Measured, us per call in a graph, decode /
-// tensor cores at 5 and 8 tokens (B3): 1024 x 1024, 1 plane 10.4 / 9.5, 11.0 / 9.2; 2560 x 2560, 1 plane 14.3 / 11.9,
-// 15.3 / 11.5; 6912 x 2560, 3 planes 22.1 / 17.6, 22.8 / 17.6; 34816 x 5120, 2 planes 66 / 51, 72 / 51; D2 alike.  The
-// decode passes win only where three B3 planes meet a last wave of row tiles that is nearly empty: 20000 x 4096,
-// 3 planes (157 tiles on 148 SMs) 50 / 63.
-bool two_passes_win(const tb_backend* b, const tb_weights* w) {
+// Five to eight tokens of a device call: two chained decode passes or one tensor-core call.  The tensor cores, where the
+// caller has reserved them for this tensor and that many tokens (tb_backend_reserve): not what other tensors or calls have
+// reserved, and not how the call is launched, decides.  Measured, us per call in a graph, decode / tensor cores at 5 and 8
+// tokens (B3): 2560 x 2560, 1 plane 14.3 / 11.9, 15.3 / 11.5; 6912 x 2560, 3 planes 22.1 / 17.6, 22.8 / 17.6; 34816 x 5120, 2 planes
+// 66 / 51, 72 / 51; D2 alike.  The decode passes stay
+//   * up to 768 columns: they build their tables themselves and so share no scratch with calls on other streams, which a
+//     tensor-core call does (it would take 8.5 us for 11.4 at 2560 x 512, 1 plane; called without a graph 11.7 for 12.4);
+//   * up to 1,024 columns with up to 2,048 rows, or with a norm, which the tensor cores need a launch more for: with dependent
+//     launch 1024 x 1024, D2, 1 plane 7.6 / 9.0, 2048 rows 8.6 / 9.0, but 2816 rows 9.6 / 8.8 (B3 8.8 / 9.5, 9.5 / 9.6, 10.2 / 9.4);
+//   * where three B3 planes meet a last wave of row tiles that is nearly empty: 20000 x 4096, 3 planes (157 tiles on 148 SMs) 50 / 63.
+bool five_to_eight_on_tensor_cores(const tb_backend* b, const tb_weights* w, uint32_t m, bool norm) {
+  if (m <= 4 || m > 8 || m > w->reserved_m) return false;
+  if (w->k <= 768 || (w->k <= 1024 && (norm || w->n <= 2048))) return false;
   const uint64_t sms = uint64_t(b->prop.multiProcessorCount), tiles = (w->n + 127) / 128, slots = (tiles + sms - 1) / sms * sms;
-  return w->uniform_planes == 3 && w->codec == tbf::kB3 && tiles > sms && tiles * 100 < slots * 55;
+  return !(w->uniform_planes == 3 && w->codec == tbf::kB3 && tiles > sms && tiles * 100 < slots * 55);
 }
 bool takes_tensor_cores(const tb_backend* b, const tb_weights* w, uint32_t m, uint32_t flags, uint32_t decode_limit = 8) {
   if (flags & TB_FWD_FORCE_PREFILL) return true;
@@ -539,16 +546,11 @@ tb_status forward_dev(tb_backend* b, const tb_weights* w, const tb_forward_args&
     fill_receipt(w, a.m, dtype_size(a.x_dtype), dtype_size(a.y_dtype), 0, ex.norm_weight ? 4 : 3, receipt);
     return TB_OK;
   }
-  // Up to four tokens one decode pass, from nine on the tensor cores.  Measured with flushed caches, us, decode /
-  // tensor cores at 4 tokens: 6912 x 2560, 3 planes 23.5 / 23.5; 2560 x 2560, 1 plane 15.6 / 19.4; 34816 x 5120, 2 planes
-  // 48 / 60.  In between the tensor cores too (see two_passes_win), if what they need is reserved: a caller that has
-  // reserved nothing keeps the two decode passes, and so do the host calls, whose copies outweigh the difference, and rows
-  // of up to 1,024 columns where a norm or programmatic dependent launch goes with them.
-  bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags);
-  if (device_call && !want_prefill && a.m > 4 && !(a.flags & TB_FWD_FORCE_DECODE) && !two_passes_win(b, w))
-    want_prefill = tb_prefill_supported(w, a.m) && b->q.cap >= tb_prefill_scratch_bytes(w, a.m) &&
-                   (!ex.norm_weight || b->norm.cap >= size_t(a.m) * w->k * 4) &&
-                   !((ex.norm_weight || (a.flags & TB_FWD_PDL)) && w->k <= 1024);
+  // Up to four tokens one decode pass, from nine on the tensor cores; in between see five_to_eight_on_tensor_cores (host calls
+  // and stacks keep the decode passes).  Measured with flushed caches, us, decode / tensor cores at 4 tokens: 6912 x 2560, 3
+  // planes 23.5 / 23.5; 2560 x 2560, 1 plane 15.6 / 19.4; 34816 x 5120, 2 planes 48 / 60.
+  const bool want_prefill = takes_tensor_cores(b, w, a.m, a.flags) ||
+                            (device_call && !(a.flags & TB_FWD_FORCE_DECODE) && five_to_eight_on_tensor_cores(b, w, a.m, ex.norm_weight != nullptr));
   uint32_t extra_launches = 0;
   // The decode kernel normalises inside its table builder.  Every other route (the tensor-core
   // kernel, tables from the preparation kernel) takes rows normalised by a kernel of its own; the
@@ -837,7 +839,10 @@ extern "C" tb_status tb_backend_reserve(tb_backend* b, const tb_weights* w, uint
   if (tb_status s = use_device(b)) return s;
   if (tb_status s = reserve_prefill(b, w, max_m)) return s;
   // normalised rows of calls of five to eight tokens (see forward_dev)
-  if (max_m > 4 && w->fast && tb_prefill_supported(w, max_m)) return ensure(b, &b->norm, size_t(std::min(max_m, 8u)) * w->k * 4);
+  if (max_m > 4 && w->fast && tb_prefill_supported(w, max_m)) {
+    if (tb_status s = ensure(b, &b->norm, size_t(std::min(max_m, 8u)) * w->k * 4)) return s;
+    w->reserved_m = std::max(w->reserved_m, max_m);
+  }
   return TB_OK;
 }
 

@@ -88,6 +88,8 @@ struct tb_weights {
   uint8_t* d_meta = nullptr;     // map bytes followed by LE u32 rank prefixes
   uint32_t* d_tile_rank = nullptr;  // planes before each tile (ragged tensors only)
   DecodePlan plan;
+  // most tokens that tb_backend_reserve was called for (0: never, or the tensor-core kernel does not take the tensor)
+  mutable uint32_t reserved_m = 0;
 };
 
 void tb_set_error(const std::string& message);
