@@ -834,7 +834,8 @@ def device_receipt(backend, resident, x, y, flags=0):
 
 @pytest.mark.parametrize("codec", [SaltV2Codec.B3, SaltV2Codec.D2])
 @pytest.mark.parametrize("n,k,planes,tensor_cores", [(4096, 768, 1, False), (2048, 1024, 2, False), (2049, 1024, 2, True), (300, 1280, 2, True),
-                                                     (18944, 1792, 3, True), (18945, 1792, 3, None)])
+                                                     (18944, 1792, 3, True), (18945, 1792, 3, None), (18945, 1536, 3, True), (23937, 1792, 3, True),
+                                                     (18945, 6144, 2, None), (18945, 5888, 2, True)])
 def test_kernel_of_five_to_eight_tokens_follows_the_tensors_own_reservation(codec, n, k, planes, tensor_cores):
     """The kernel of a call of five to eight tokens depends on the tensor and on what was reserved for it: not on other
     tensors' reservations, host calls or launch flags.  None: only B3 keeps the decode passes (a second wave of row

@@ -454,12 +454,19 @@ bool decode_fits(const tb_backend* b, const tb_weights* w, uint32_t m) {
 //     tensor-core call does (it would take 8.5 us for 11.4 at 2560 x 512, 1 plane; called without a graph 11.7 for 12.4);
 //   * up to 1,024 columns with up to 2,048 rows, or with a norm, which the tensor cores need a launch more for: with dependent
 //     launch 1024 x 1024, D2, 1 plane 7.6 / 9.0, 2048 rows 8.6 / 9.0, but 2816 rows 9.6 / 8.8 (B3 8.8 / 9.5, 9.5 / 9.6, 10.2 / 9.4);
-//   * where three B3 planes meet a last wave of row tiles that is nearly empty: 20000 x 4096, 3 planes (157 tiles on 148 SMs) 50 / 63.
+//   * where long B3 rows meet a second wave of row tiles that is nearly empty: 3 planes, 2,048 columns, 149 / 172 / 184 / 192 / 208
+//     tiles at 5 tokens 30.9 / 36.0, 33.4 / 35.4, 33.8 / 35.3, 35.5 / 35.2, 37.3 / 35.5, and 4,096 columns, 149 / 184 / 208 tiles
+//     52 / 64, 57 / 64, 66 / 64 (at 8 tokens 56 / 65, 61 / 64, 70 / 64), but 1,536 columns, 152 tiles, 8 tokens 29.6 / 28.1; 2 planes,
+//     8,192 columns, 152 / 162 / 176 tiles 68 / 79, 71 / 80, 76 / 80 (at 8 tokens 73 / 81, 76 / 80, 81 / 80), 6,144 columns
+//     59 / 61, 60 / 60, 65 / 61, but 3,072 columns, 152 tiles 40 / 34.
 bool five_to_eight_on_tensor_cores(const tb_backend* b, const tb_weights* w, uint32_t m, bool norm) {
   if (m <= 4 || m > 8 || m > w->reserved_m) return false;
   if (w->k <= 768 || (w->k <= 1024 && (norm || w->n <= 2048))) return false;
-  const uint64_t sms = uint64_t(b->prop.multiProcessorCount), tiles = (w->n + 127) / 128, slots = (tiles + sms - 1) / sms * sms;
-  return !(w->uniform_planes == 3 && w->codec == tbf::kB3 && tiles > sms && tiles * 100 < slots * 55);
+  const uint64_t sms = uint64_t(b->prop.multiProcessorCount), tiles = (w->n + 127) / 128;
+  if (w->codec != tbf::kB3 || tiles <= sms) return true;
+  if (w->uniform_planes == 3) return w->k < 1792 || tiles * 100 > sms * 127;
+  if (w->uniform_planes == 2) return w->k < 6144 || tiles * 100 > sms * 110;
+  return true;
 }
 bool takes_tensor_cores(const tb_backend* b, const tb_weights* w, uint32_t m, uint32_t flags, uint32_t decode_limit = 8) {
   if (flags & TB_FWD_FORCE_PREFILL) return true;
