@@ -904,16 +904,19 @@ uint32_t tile_tokens(const tb_weights* w, uint32_t m, uint32_t sm_count) {
   return half == whole || (2 * half <= 3 * whole && tile_planes <= 40) || tile_planes <= 4 ? 128 : 256;
 }
 // K splits of an output tile, for token tiles of up to 128: as many as keep every CTA of one wave busy, at most one
-// per tile column.  A 128-token tile passes 64 KB of sums through memory per part, about 6 us, or the time of
-// seven tile-planes: it is split where at least kWorthTilePlanes are saved.  Measured, whole / split, us: 5120 x 5120,
-// 2 planes, 100 tokens (26 saved) 44.5 / 28.3; 2560 x 2560, 3 planes, 128 tokens (24) 35.3 / 25.6; 2560 x 6912, 1 plane,
-// 200 tokens (18) 32.1 / 24.6; but 8192 x 2048, 1 plane, 128 tokens (4) 16.3 / 17.6.
-constexpr uint32_t kWorthTilePlanes = 10;
+// per tile column.  A 128-token tile passes 64 KB of sums through memory per part and the last CTA adds them up, about
+// 6 us with two or three parts: it is split where that saves a CTA ten tile-planes, with six parts twelve, with
+// more 14.  Measured, whole / split, us: two and three parts, 4 and 5 saved 16.4 / 17.5, 15.8 / 17.8 (6912 x 1024, 2 planes,
+// and 5120 x 2048, 1 plane, 100 tokens), 10 saved 23.3 / 21.1, 28.6 / 25.2 (5120 x 2048, 2 planes, 128; 2560 x 5120, 1 plane, 300),
+// 18 saved 42.3 / 31.4 (8192 x 3072, 3 planes, 100); six parts, 10 saved 20.6 / 21.2, 13 saved 23.9 / 22.4 (1024 x 3072 and 4096,
+// 1 plane, 300); seven, 13 saved 21.6 / 22.8, 16 saved 26.0 / 23.9 (2560 x 4096, 1 plane, and 2560, 2 planes, 128); eight, 7 saved
+// 15.3 / 20.0, 14 saved 21.8 / 20.5 (1024 x 2048, 1 plane, 128, and 2 planes, 100).
 uint32_t splits_of(const tb_weights* w, uint32_t m, uint32_t tt, uint32_t sm_count) {
   const uint32_t tpr = uint32_t(w->k / 256), out_tiles = uint32_t((w->n + kRows - 1) / kRows) * ((m + tt - 1) / tt);
   if (tt > 128 || out_tiles >= sm_count || out_tiles > kMaxSplitTiles) return 1;
   const uint32_t splits = std::max(1u, std::min(std::min(sm_count / out_tiles, tpr), 8u));
-  if (tt == 128 && (tpr - (tpr + splits - 1) / splits) * w->uniform_planes < kWorthTilePlanes) return 1;
+  const uint32_t worth = std::max(10u, std::min(2u * splits, 14u));
+  if (tt == 128 && (tpr - (tpr + splits - 1) / splits) * w->uniform_planes < worth) return 1;
   return splits;
 }
 
