@@ -9,7 +9,10 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import math
 import threading
+import weakref
+from collections import deque
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -154,24 +157,59 @@ class _HostBuffer:
 class _HostPool:
     """Output arrays of the host-pointer calls in pinned memory: the GPU copies straight into them, and no page of
     theirs is touched for the first time.  Bound by those copies and page faults before: fp32 activations, 32 tokens,
-    8192 x 2048 (1 MB out) 277 -> 106 us a call; 26 layers of 6912 x 2560 at one token (360 KB out) 156 -> 130 us.
+    8192 x 2048 (1 MB out) 268 -> 104 us a call; 26 layers of 6912 x 2560 at one token (360 KB out) 162 -> 134 us.
 
-    Sizes are powers of two; at most ``LIMIT`` bytes are pinned at a time, in use and idle together; beyond that
-    arrays come from ordinary memory, as small ones do.
+    Pinning memory costs more than it saves in one call (0.3 ms for 512 KB, 1.3 ms for 1 MB), so it is done only for a caller
+    that drops its results (see ``output``): one that keeps all of 60 paid 466 us a call of those layers while every call
+    pinned, and pays 159 us now.  Sizes are powers of two; at most ``LIMIT`` bytes are pinned at a time, in use and idle
+    together; beyond that arrays come from ordinary memory, as small ones do.
     """
 
     LIMIT = 256 << 20
     SMALLEST = 16 << 10   # below, a bounce copy and a few page faults cost less than the bookkeeping
+    EVICT_EVERY = 64      # calls between two that free idle buffers to make room, so that sizes which do not all fit don't pin in turn
 
     def __init__(self, lib, backend_handle):
         self._L, self._backend = lib, backend_handle
         self._lock = threading.RLock()   # give_back may run in a collection inside array()
         self._idle: dict = {}
+        self._plain: dict = {}           # size -> the last arrays of ordinary memory, weakly
         self._pinned = 0
+        self._calls = 0
+        self._evicted = -self.EVICT_EVERY
         self._closed = False
 
-    def array(self, shape, dtype) -> np.ndarray:
-        need = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+    @staticmethod
+    def _size(shape, dtype) -> int:
+        return math.prod(shape) * np.dtype(dtype).itemsize
+
+    def output(self, shape, dtype) -> np.ndarray:
+        """The array a call returns.  Pinned where an idle buffer fits, or where one of the last two ordinary arrays of
+        the size is gone: a caller that drops its results, or keeps the last one, has two buffers pinned after four calls;
+        one that keeps them all has ordinary memory throughout."""
+        need = self._size(shape, dtype)
+        if need < self.SMALLEST:
+            return np.empty(shape, dtype)
+        size = 1 << (need - 1).bit_length()
+        with self._lock:
+            self._calls += 1
+            idle = self._idle.get(size)
+            if idle:
+                return np.asarray(_HostBuffer(self, idle.pop(), size, shape, dtype))
+            plain = self._plain.setdefault(size, deque(maxlen=2))
+            gone = next((r for r in plain if r() is None), None)
+            if gone is not None:
+                plain.remove(gone)
+                may_evict = self._calls - self._evicted >= self.EVICT_EVERY
+                if may_evict and self._pinned + size > self.LIMIT:
+                    self._evicted = self._calls
+                return self.array(shape, dtype, may_evict)
+            out = np.empty(shape, dtype)
+            plain.append(weakref.ref(out))
+            return out
+
+    def array(self, shape, dtype, may_evict: bool = True) -> np.ndarray:
+        need = self._size(shape, dtype)
         if need < self.SMALLEST:
             return np.empty(shape, dtype)
         size = 1 << (need - 1).bit_length()
@@ -179,7 +217,7 @@ class _HostPool:
             idle = self._idle.get(size)
             ptr = idle.pop() if idle else None
             if ptr is None:
-                if self._pinned + size > self.LIMIT:
+                if self._pinned + size > self.LIMIT and may_evict:
                     self._free_idle()
                 if self._closed or self._pinned + size > self.LIMIT:
                     return np.empty(shape, dtype)
@@ -328,7 +366,7 @@ class B200Backend:
         act = np.ascontiguousarray(activation, np.float32)
         if act.size != m * t.columns:
             raise ShapeMismatch(f"shape mismatch: expected {m * t.columns}, got {act.size}")
-        out = self._host.array((m, t.rows), np.float32)
+        out = self._host.output((m, t.rows), np.float32)
         r = _lib.Receipt()
         check(fn(self._h, t._h, _ptr(act), C.c_uint32(m), _ptr(out), C.byref(r)))
         return SaltV2Forward(out, self._receipt(r, mode))
@@ -368,7 +406,7 @@ class B200Backend:
             xd = _lib.TB_F32
         if xa.size != m * k:
             raise ShapeMismatch(f"shape mismatch: expected {m * k}, got {xa.size}")
-        y = self._host.array((m, n), np.float32 if y_dtype == "f32" else np.uint16)
+        y = self._host.output((m, n), np.float32 if y_dtype == "f32" else np.uint16)
         yd = _lib.TB_F32 if y_dtype == "f32" else _lib.TB_BF16
         planes = int(t.info["planes_uniform"])
         acc = np.zeros((m, n, k // 128, max(planes, 1)), np.int32) if dump else None
@@ -478,7 +516,7 @@ class LinearStack:
         layers must all read the stack input and share n."""
         xa = np.ascontiguousarray(x, np.uint16 if x_is_bf16 else np.float32)
         n = self._weights[0].rows
-        y = self._backend._host.array((len(self._weights), m, n), np.uint16)
+        y = self._backend._host.output((len(self._weights), m, n), np.uint16)
         check(self._backend._L.tb_stack_forward_host(self._h, _ptr(xa), _lib.TB_BF16 if x_is_bf16 else _lib.TB_F32, C.c_uint32(m), _ptr(y),
                                             C.c_uint32(flags)))
         return y
