@@ -212,3 +212,49 @@ def test_two_gpu_tensor_parallel_matches_unsharded_reference(codec, use_peer):
             for m, (err_col, err_row, absmax_ok) in results[rank].items():
                 assert err_col <= 1e-5 and err_row <= 1e-5, (rank, m, err_col, err_row)
                 assert absmax_ok, (rank, m)
+
+
+def unaligned_main(rank, world, port, results):
+    """Gated row shard whose operands lie 4 bytes past a 16-byte boundary on rank 1 only: both ranks take the same route,
+    and the result is that of aligned operands."""
+    import torch.distributed as dist
+    from tritium_b200 import B200Backend, tp
+    from tritium_b200.format import SaltV2Codec
+    from tritium_b200.synth import make_tensor
+
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    torch.cuda.set_device(rank)
+    dist.init_process_group("nccl", rank=rank, world_size=world, device_id=torch.device("cuda", rank))
+    try:
+        backend = B200Backend(rank)
+        comm = tp.PeerComm(backend, rank, world, slot_bytes=64 * 512 * 4, slots=8)
+        ex = tp.CudaExecutor(backend, comm=comm)
+        out = {}
+        for m, n, k in [(1, 256, 10240), (4, 256, 2048), (7, 200, 1536)]:   # 20 and 16 pairs, two passes
+            row = tp.TPLinear(ex, make_tensor("down", n, k, 1, seed=m), SaltV2Codec.B3, "row", rank, world, max_m=m, act_dtype=torch.float32)
+            torch.manual_seed(rank)
+            row.x.normal_()
+            up = torch.randn_like(row.x)
+            comm.block_linear_fused(row.handle, row.slot_absmax, row.slot_y, row.x[:m], row.y[:m], relu2_up=up[:m])
+            want = row.y[:m].clone()
+            past = [torch.zeros(t.numel() + 4, device="cuda") for t in (row.x, up)]
+            moved = [p[rank:rank + t.numel()].view_as(t).copy_(t) for p, t in zip(past, (row.x, up))]
+            comm.block_linear_fused(row.handle, row.slot_absmax, row.slot_y, moved[0][:m], row.y[:m], relu2_up=moved[1][:m])
+            torch.cuda.synchronize()
+            backend.check()
+            out[m] = bool(torch.equal(row.y[:m], want))
+        results[rank] = out
+        comm.close()
+    finally:
+        dist.destroy_process_group()
+
+
+def test_two_gpu_operands_that_are_unaligned_on_one_rank():
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    import torch.multiprocessing as mp
+    with mp.Manager() as manager:
+        results = manager.dict()
+        mp.spawn(unaligned_main, args=(2, free_port(), results), nprocs=2, join=True)
+        for rank in range(2):
+            assert all(results[rank].values()), (rank, dict(results[rank]))

@@ -832,8 +832,28 @@ tb_status forward_tp(tb_backend* b, const tb_weights* w, tb_comm* comm, uint32_t
     d.residual = ex.residual ? ex.residual + size_t(m0) * w->n : nullptr;
     // Small tables: ONE launch (absmax exchange in the table builder, output sum in the epilogue).
     // Large tables: the preparation kernel exchanges the absmax, the decode kernel sums the outputs.
-    d.fused = tb_decode_builds_tables(w, mc, d.x);
-    if (!d.fused) TB_CUDA(tb_launch_prepare(d, st), "launch prepare");
+    // The ranks must agree on which, so the tensor's shape decides alone; rows that are not 16-byte aligned, on
+    // this rank, are copied into the scratch that a launch with its own tables leaves free.
+    d.fused = tb_decode_builds_tables(w, mc, nullptr);
+    if (d.fused) {
+      uint8_t* free_scratch = static_cast<uint8_t*>(b->d_prep);   // 2 MB; the rows of a pass take 32 KB at most
+      cudaError_t copied = cudaSuccess;
+      const auto align_rows = [&](const void* rows, size_t elem) -> const void* {
+        if (!rows || (reinterpret_cast<uintptr_t>(rows) & 15u) == 0) return rows;
+        const size_t bytes = size_t(mc) * w->k * elem;
+        uint8_t* copy = free_scratch;
+        free_scratch += (bytes + 255) & ~size_t(255);
+        copied = cudaMemcpyAsync(copy, rows, bytes, cudaMemcpyDeviceToDevice, st);
+        d.pdl = false;   // dependent launch is between kernels
+        return copied == cudaSuccess ? copy : nullptr;
+      };
+      d.x = align_rows(d.x, dtype_size(x_dtype));
+      TB_CUDA(copied, "align activations");
+      d.relu2_up = static_cast<const float*>(align_rows(d.relu2_up, 4));
+      TB_CUDA(copied, "align the gate's operand");
+    } else {
+      TB_CUDA(tb_launch_prepare(d, st), "launch prepare");
+    }
     TB_CUDA(tb_launch_decode(d, b->prop.multiProcessorCount, b->max_smem_optin, st), "launch decode");
   }
   return TB_OK;
