@@ -869,3 +869,18 @@ def test_kernel_of_five_to_eight_tokens_follows_the_tensors_own_reservation(code
     for h in (w, other):
         h.free()
     b.close()
+
+
+@pytest.mark.parametrize("codec,k,m,launches", [(SaltV2Codec.D2, 3072, 1, 1), (SaltV2Codec.D2, 3328, 1, 2), (SaltV2Codec.D2, 1536, 2, 1),
+                                                (SaltV2Codec.D2, 1792, 2, 2), (SaltV2Codec.D2, 768, 4, 1), (SaltV2Codec.D2, 1024, 3, 2),
+                                                (SaltV2Codec.B3, 8192, 1, 1), (SaltV2Codec.B3, 8448, 1, 2), (SaltV2Codec.B3, 4096, 2, 1),
+                                                (SaltV2Codec.B3, 4352, 2, 2), (SaltV2Codec.B3, 1024, 3, 1), (SaltV2Codec.B3, 1280, 4, 2)])
+def test_tables_on_both_sides_of_the_builders_limit(backend, codec, k, m, launches):
+    """The largest tables that the decode kernel builds itself (one launch; D2 12 pairs, B3 32, with the four-token
+    layout 16) and the smallest that the preparation kernel builds (two), each against the oracle."""
+    import torch
+    prod, _ = uniform_pair(20, k, 1, seed=k + m)
+    resident = backend.upload_salt_v2(prod, codec)
+    y = torch.zeros(m, 20, device="cuda")
+    assert device_receipt(backend, resident, torch.zeros(m, k, device="cuda"), y).launches == launches
+    test_activation_tables_where_their_passes_end(backend, codec, k, m)

@@ -490,10 +490,9 @@ __device__ __forceinline__ void clear_tables(const DecodeParams& p, uint8_t* sme
 //
 // Bound by latency and by instruction fetch (the code runs once per launch, from a cold cache), so it is
 // kept short: every activation is loaded once and stays in registers up to kChunkPairs pairs, loops stay
-// rolled, packed arithmetic builds the entries.  The form before (eight activations per lane, loaded once
-// for the absmax and again for the codes, unrolled; byte arithmetic for the entries) took 8,700 clocks for
-// ten pairs, 4,650 of them in the straight-line quantisation.  2560 x 2560, one plane, 1 token: 7.8 -> 5.7 us
-// per launch; 13824 x 2560: 10.6 -> 8.1; 32 launches of a decoder's layers, norms and residuals included: 352 -> 267 us.
+// rolled, packed arithmetic builds the entries: about 3,700 clocks for ten pairs (8,700 with two readings and
+// unrolled loops).  2560 x 2560, one plane, 1 token 5.7 us per launch (7.8); 13824 x 2560 8.1 (10.6); 32 launches of a
+// decoder's layers, norms and residuals included, 267 us (352).
 //
 // Codes are staged with 128 added (u = x + 128).  Work item of the entry construction = one packed word w
 // of one (tile column, token, scale group): the 20 (B3) or 16 (D2) activations that meet the word's
@@ -1295,11 +1294,16 @@ bool tb_decode_supported(const tb_weights* w, uint32_t m, int max_smem, size_t* 
 size_t tb_decode_scratch_bytes(const tb_weights* w, uint32_t m) { return table_layout(w, m).total; }
 
 bool tb_decode_builds_tables(const tb_weights* w, uint32_t m, const void* x) {
-  // Every CTA quantises and lays out all (tile column, token) pairs.  Measured on B200, us per call in a graph,
-  // in the kernel / preparation kernel in front: one token, 20 pairs 30.7 / 30.8 (34816 x 5120) and 11.2 / 10.9
-  // (5120 x 5120), 27 pairs 9.2 / 9.7 (2560 x 6912), 68 pairs 26.5 / 21.8 (5120 x 17408); four tokens, 40 pairs
-  // 15.2 / 12.1, 80 pairs 18.1 / 12.1.  Level at 20 pairs, where the second launch costs the host 2 us besides; a
-  // four-token table has twice the entries per pair and goes by one pass of the builder.
+  // Every CTA quantises and lays out all (tile column, token) pairs.  Measured on B200, us a call, in the kernel / by the
+  // preparation kernel in front, B3.  In a graph, one token: 20 pairs 9.9 / 10.0, 24.1 / 24.3 (2560 and 20480 x 5120, 2 planes),
+  // 27 pairs 9.4 / 10.0 (2560 x 6912), 28 pairs 11.7 / 11.5, 21.7 / 22.9 (2560 x 7168, 2 planes, 8192 x 7168, 3 planes), 32 pairs
+  // 10.9 / 11.2, 19.7 / 18.8 (2560 x 8192, 1 plane, 8192 x 8192, 2 planes), 68 pairs 26.5 / 21.8 (5120 x 17408).  Two tokens: 16 pairs
+  // 5.9 / 6.9, 20 pairs 7.6 / 7.5, 24 pairs 7.8 / 7.5, 32 pairs 8.6 / 7.9 (2560 rows, 1 plane).  The preparation kernel is a
+  // launch more: without a graph the same calls take 2 us less with the builder up to the limit (2560 x 8192 12.4 / 15.5,
+  // 2560 x 4096 at two tokens 10.3 / 12.3), and behind a norm, which the builder takes along, decoder layers of 3,072
+  // columns at two tokens 179 / 197, of 7,168 at one 141 / 161.  So the limit stands at 32 pairs, where a graph of
+  // two-token calls without a norm loses up to 14 % (dependent launches 23 %).  Four tokens: 16 pairs 6.3 / 6.9,
+  // 8.0 / 8.9 (2560 and 8192 x 1024, 2 planes), 40 pairs 15.2 / 12.1, 80 pairs 18.1 / 12.1; twice the entries per pair.
   // D2 leaves the launch less time for the builder to hide in: 25 pairs 19.0 / 18.5 (30848 x 6400, one token), layers of
   // 1,024 columns at 8 tokens (16 pairs) 160 / 152 us, where B3 takes 166 / 176.
   const uint32_t mk = layout_tokens(m), pairs = uint32_t(w->k / 256) * mk;
