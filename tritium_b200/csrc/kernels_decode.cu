@@ -56,8 +56,8 @@ struct DecodeParams {
   const uint8_t* payload; const uint16_t* scales;   // single layer (layers == nullptr)
   const TbLayerDesc* layers; uint32_t layer_count; uint32_t y_layer_stride;   // grouped launch: outputs [layer][m][n]
   const uint8_t* tables; uint32_t table_bytes;   // z tables | accumulator start values | token scales
-  // fused prologue (kernels with BUILD): the CTA quantises x and builds its tables itself
-  const void* x; const float* act_scale_in; const float* act_absmax_in; uint32_t x_dtype;
+  // fused prologue (fused != 0, kernels with BUILD): the CTA quantises x and builds its tables itself
+  const void* x; const float* act_scale_in; const float* act_absmax_in; uint32_t x_dtype, fused;
   // fused RMSNorm in front of the quantiser (fused launches only; null = none) and `residual + y`
   // behind the token scale (fp32, indexed like y; null = none)
   const float* norm_weight; float norm_eps; uint32_t norm_zero_centered;
@@ -768,12 +768,13 @@ __device__ __forceinline__ void build_tables(const DecodeParams& p, uint8_t* sme
 // ---------------------------------------------------------------- the kernel
 // M: token columns the tables are laid out for (1, 2 or 4; p.m <= M tokens are valid).
 // SETS: blocks of 16 row-planes in one row block (rows_per_stage * PLANES / 16).
-// BUILD: the kernel builds its activation tables itself (else it reads those of prepare_kernel).  Two kernels,
+// BUILD: the kernel can build its activation tables itself (else it reads those of prepare_kernel).  Two kernels,
 // because the builder takes 90 to 96 registers per thread where the main loop of small row blocks takes 70 to 77:
 // without it the CTAs of two launches leave the registers that a preparation kernel needs to start beside
 // them, and a chain of dependent launches overlaps.  One kernel for both / two, us a call of such a chain: 2688 x 2048,
 // 2 planes, 3 tokens, B3 7.3 / 6.1; 11264 x 2048, 2 planes, 4 tokens, D2 9.6 / 8.4; four decoder layers of 2,048 columns,
-// 2 planes, 4 tokens, B3 172 / 158.
+// 2 planes, 4 tokens, B3 172 / 158.  The kernel with the builder keeps the other branch too: the main loop is compiled
+// better with it (34816 x 5120, 2 planes, 1 token 33.3 us, 33.5 without; decoder layers 266.5, 268.0).
 template <int CODEC, int PLANES, int M, int SETS, bool BUILD>
 __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams p) {
   using T = Traits<CODEC>;
@@ -815,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   // builds its own tables shares no scratch with its neighbours, so it raises the trigger at
   // once.  A launch that waits for tables in global scratch raises it only after that wait, so
   // that a later launch which shares the tables (and does not wait) cannot outrun them.
-  if (p.pdl && (BUILD || !p.wait_tables)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.pdl && ((BUILD && p.fused) || !p.wait_tables)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   const uint32_t total_blocks = p.blocks * p.layer_count;
   const uint32_t my_blocks = blockIdx.x < total_blocks ? (total_blocks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -971,7 +972,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
   }
 
   // -------------------------------------------------- consumers: activation tables
-  if constexpr (BUILD) {
+  if (BUILD && p.fused) {
     clear_tables(p, smem, tid);
     consumer_sync();
     // x may be the previous kernel's output: wait for it (the weight stream is already running)
@@ -1375,7 +1376,7 @@ cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cu
     if (a.comm_absmax && !a.comm_y) return cudaErrorInvalidValue;
     if (a.comm_y && a.comm_y->world > 1 && !a.comm_absmax && !a.act_absmax_in && a.x_dtype != TB_I8) return cudaErrorInvalidValue;
     if (a.x_dtype == TB_I8 && !a.act_scale_in) return cudaErrorInvalidValue;
-    p.x = a.x; p.act_scale_in = a.act_scale_in; p.act_absmax_in = a.act_absmax_in; p.x_dtype = uint32_t(a.x_dtype);
+    p.fused = 1; p.x = a.x; p.act_scale_in = a.act_scale_in; p.act_absmax_in = a.act_absmax_in; p.x_dtype = uint32_t(a.x_dtype);
     if (a.relu2_up) {
       if (a.x_dtype != TB_F32 || (reinterpret_cast<uintptr_t>(a.relu2_up) & 15u) || a.norm_weight) return cudaErrorInvalidValue;
       p.relu2_up = a.relu2_up;
