@@ -768,13 +768,15 @@ __device__ __forceinline__ void build_tables(const DecodeParams& p, uint8_t* sme
 // ---------------------------------------------------------------- the kernel
 // M: token columns the tables are laid out for (1, 2 or 4; p.m <= M tokens are valid).
 // SETS: blocks of 16 row-planes in one row block (rows_per_stage * PLANES / 16).
-// BUILD: the kernel can build its activation tables itself (else it reads those of prepare_kernel).  Two kernels,
-// because the builder takes 90 to 96 registers per thread where the main loop of small row blocks takes 70 to 77:
-// without it the CTAs of two launches leave the registers that a preparation kernel needs to start beside
-// them, and a chain of dependent launches overlaps.  One kernel for both / two, us a call of such a chain: 2688 x 2048,
+// BUILD: the kernel can build its activation tables itself, else it only reads those of prepare_kernel.  Four tokens
+// have a kernel of each kind, because the builder takes 91 to 96 registers per thread where the main loop of small row
+// blocks takes 70: without it the CTAs of two launches leave the registers that a preparation kernel needs to start
+// beside them, and a chain of dependent launches overlaps.  One kernel for both / two, us a call of such a chain: 2688 x 2048,
 // 2 planes, 3 tokens, B3 7.3 / 6.1; 11264 x 2048, 2 planes, 4 tokens, D2 9.6 / 8.4; four decoder layers of 2,048 columns,
-// 2 planes, 4 tokens, B3 172 / 158.  The kernel with the builder keeps the other branch too: the main loop is compiled
-// better with it (34816 x 5120, 2 planes, 1 token 33.3 us, 33.5 without; decoder layers 266.5, 268.0).
+// 2 planes, 4 tokens, B3 172 / 158.  One and two tokens have one kernel: few of their launches have prepared tables, and chains
+// that mix both kinds lose (3 layers of 1,024 columns, ffn 9,472, 1 token 55.8 / 57.6; of 2,304, ffn 8,448 97.5 / 99.3).  The
+// kernel with the builder keeps the other branch in any case: the main loop is compiled better with it (34816 x 5120,
+// 2 planes, 1 token 33.3 us, 33.5 without; decoder layers 266.5, 268.0).
 template <int CODEC, int PLANES, int M, int SETS, bool BUILD>
 __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams p) {
   using T = Traits<CODEC>;
@@ -1343,24 +1345,21 @@ cudaError_t tb_launch_prepare(const DecodeArgs& a, cudaStream_t stream) {
 }
 
 using DecodeKernel = void (*)(const DecodeParams);
-template <int CODEC, int PLANES, int SETS, bool BUILD> DecodeKernel pick_tokens(uint32_t mk) {
-  return mk == 1   ? decode_kernel<CODEC, PLANES, 1, SETS, BUILD>
-         : mk == 2 ? decode_kernel<CODEC, PLANES, 2, SETS, BUILD>
-                   : decode_kernel<CODEC, PLANES, 4, SETS, BUILD>;
+template <int CODEC, int PLANES, int SETS> DecodeKernel pick_tokens(uint32_t mk, bool build) {
+  return mk == 1   ? decode_kernel<CODEC, PLANES, 1, SETS, true>
+         : mk == 2 ? decode_kernel<CODEC, PLANES, 2, SETS, true>
+         : build   ? decode_kernel<CODEC, PLANES, 4, SETS, true>
+                   : decode_kernel<CODEC, PLANES, 4, SETS, false>;
 }
-template <int CODEC, int PLANES, bool BUILD> DecodeKernel pick_sets(uint32_t sets, uint32_t mk) {
-  return sets == 1   ? pick_tokens<CODEC, PLANES, 1, BUILD>(mk)
-         : sets == 2 ? pick_tokens<CODEC, PLANES, 2, BUILD>(mk)
-                     : pick_tokens<CODEC, PLANES, 4, BUILD>(mk);
+template <int CODEC, int PLANES> DecodeKernel pick_sets(uint32_t sets, uint32_t mk, bool build) {
+  return sets == 1   ? pick_tokens<CODEC, PLANES, 1>(mk, build)
+         : sets == 2 ? pick_tokens<CODEC, PLANES, 2>(mk, build)
+                     : pick_tokens<CODEC, PLANES, 4>(mk, build);
 }
-template <int CODEC, bool BUILD> DecodeKernel pick_planes(uint32_t planes, uint32_t sets, uint32_t mk) {
-  return planes == 1   ? pick_sets<CODEC, 1, BUILD>(sets, mk)
-         : planes == 2 ? pick_sets<CODEC, 2, BUILD>(sets, mk)
-                       : pick_tokens<CODEC, 3, 3, BUILD>(mk);
-}
-DecodeKernel pick_kernel(int codec, uint32_t planes, uint32_t sets, uint32_t mk, bool build) {
-  if (codec == tbf::kB3) return build ? pick_planes<tbf::kB3, true>(planes, sets, mk) : pick_planes<tbf::kB3, false>(planes, sets, mk);
-  return build ? pick_planes<tbf::kD2, true>(planes, sets, mk) : pick_planes<tbf::kD2, false>(planes, sets, mk);
+template <int CODEC> DecodeKernel pick_planes(uint32_t planes, uint32_t sets, uint32_t mk, bool build) {
+  return planes == 1   ? pick_sets<CODEC, 1>(sets, mk, build)
+         : planes == 2 ? pick_sets<CODEC, 2>(sets, mk, build)
+                       : pick_tokens<CODEC, 3, 3>(mk, build);
 }
 
 cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cudaStream_t stream) {
@@ -1415,7 +1414,7 @@ cudaError_t tb_launch_decode(const DecodeArgs& a, int sm_count, int max_smem, cu
   p.wait_tables = a.tables_shared ? 0u : 1u;
   p.inject_missing_tx = a.inject_missing_tx;
   const uint32_t sets = w->plan.rows_per_stage * w->uniform_planes / 16, mk = layout_tokens(a.m);
-  DecodeKernel kernel = pick_kernel(w->codec, w->uniform_planes, sets, mk, a.fused);
+  DecodeKernel kernel = w->codec == tbf::kB3 ? pick_planes<tbf::kB3>(w->uniform_planes, sets, mk, a.fused) : pick_planes<tbf::kD2>(w->uniform_planes, sets, mk, a.fused);
   if (!kernel) return cudaErrorInvalidConfiguration;
   if (a.layers && a.layer_count > uint32_t(kMaxGroupLayers)) return cudaErrorInvalidValue;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
