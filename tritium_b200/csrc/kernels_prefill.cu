@@ -1,4 +1,4 @@
-// Tensor-core GEMM (nine tokens and more) from the packed B3 / D2 arenas on tcgen05 INT8.
+// Tensor-core GEMM (nine tokens and more, five to eight where reserved) from the packed B3 / D2 arenas on tcgen05 INT8.
 //
 //   Y[m,n] = a[m] * sum over (tile column j, plane p, group g) of s[n,j,p,g] * I[m,n,j,p,g],
 //   I = sum over the 128 trits of the group of t * q          (exact int32)

@@ -205,7 +205,7 @@ struct PrefillArgs {
   uint32_t* status;
   const float* residual = nullptr;       // [m][n] fp32, nullable: out = residual + y
   const float* relu2_up = nullptr;       // squared-ReLU gate: activation = (max(x, 0)^2) * relu2_up (x fp32)
-  uint32_t* tile_counters = nullptr;     // 256 zeroed words (launches of up to 64 tokens split K and count the splits of a tile in)
+  uint32_t* tile_counters = nullptr;     // 256 zeroed words (launches with token tiles of up to 128 split K and count the splits of a tile in)
 };
 bool tb_prefill_supported(const tb_weights* w, uint32_t m);
 // Whether the launch for `m` tokens accepts a kernel that was compiled to `launch_regs` registers per thread.
