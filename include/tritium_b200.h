@@ -193,14 +193,16 @@ tb_status tb_salt_v2_gather_rows(tb_backend* backend, const tb_weights* weights,
 #define TB_FWD_FORCE_DECODE 8u   /* streaming kernel whatever m; TB_UNSUPPORTED_FORMAT when a row block does not fit */
 #define TB_FWD_FORCE_PREFILL 16u /* tensor-core kernel whatever m */
 /* Without a force flag: up to 4 tokens take the streaming (decode) kernel, more than 8 the tensor-core
- * kernels.  5 to 8 tokens take two chained streaming passes, or the tensor cores in a device call on a tensor that
- * tb_backend_reserve was called for with at least that many tokens (short rows, and
- * a band of shapes with a nearly empty last wave of tiles, keep the passes).  The group sums are the same integers either way; the order in
- * which fp32 adds them is the kernel's, so the last bits of a call differ between the two, and between a device call and the
- * host call of the same tokens.  A tensor whose rows are too long for the streaming kernel's shared-memory ring takes the
- * tensor-core kernel at every m (so a device-pointer caller reserves with tb_backend_reserve).
- * Calls on one backend share its scratch (quantised activations, tables of long rows): calls on several streams are to be
- * ordered, or use a backend each.  Only calls whose tables the streaming kernel builds itself use none. */
+ * kernels.  5 to 8 tokens take two chained streaming passes, or the tensor cores in a device call on a
+ * tensor that tb_backend_reserve was called for with at least that many tokens (short rows, and a band of
+ * shapes with a nearly empty last wave of tiles, keep the passes; so do host calls and stacks).  The group
+ * sums are the same integers either way; the order in which fp32 adds them is the kernel's, so the last
+ * bits differ between the two, and between a device call and the host call of the same tokens.  A tensor
+ * whose rows are too long for the streaming kernel's shared-memory ring takes the tensor-core kernel at
+ * every m (so a device-pointer caller reserves with tb_backend_reserve).
+ * Calls on one backend share its scratch (quantised activations, tables of long rows): calls on several
+ * streams are to be ordered, or use a backend each.  Only calls whose tables the streaming kernel builds
+ * itself use none. */
 typedef struct tb_forward_args {
   const void* x;            /* [m,k] device */
   tb_dtype x_dtype;
